@@ -11,7 +11,7 @@ import sys
 HERE = os.path.dirname(os.path.abspath(__file__))
 SRCS = [os.path.join(HERE, "csrc", f) for f in ("gemsgpu.cu", "noalloc.cu", "peaks.cu")]
 OUT = os.path.join(HERE, "libgemsgpu.so")
-DEPS = [os.path.join(HERE, "csrc", f) for f in ("gemsgpu.cu", "noalloc.cu", "peaks.cu", "kernels.cuh", "lbfgs.cuh", "neb.cuh",
+DEPS = [os.path.join(HERE, "csrc", f) for f in ("gemsgpu.cu", "noalloc.cu", "peaks.cu", "kernels.cuh", "team.cuh", "lbfgs.cuh", "neb.cuh",
                                                              "common.cuh")] + [
     os.path.join(os.path.dirname(HERE), "include", "gemsgpu.h")]
 
@@ -19,7 +19,7 @@ NVCC_FLAGS = [
     "-O3", "-std=c++17", "-lineinfo",
     "-gencode", "arch=compute_100a,code=sm_100a",
     "-Xcompiler", "-fPIC", "-shared",
-    "--expt-relaxed-constexpr",
+    "--expt-relaxed-constexpr", "--split-compile=0",
 ]
 
 

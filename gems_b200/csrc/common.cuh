@@ -56,7 +56,9 @@ enum PREC : int { PREC_FP64 = 0, PREC_MIXED = 1 };
 // dimension, or its volume collapsed
 // ST_BONDS: a Tersoff atom has more than TS_MAXB bonds, a bond beyond list
 // slot 63, or a bond its partner's list does not hold
-enum ST : int { ST_OVERFLOW = 1, ST_LOST = 2, ST_NAN = 4, ST_BOX = 8, ST_BONDS = 16 };
+// ST_TIMEOUT: a team barrier's bounded wait ran out (the host undoes the
+// launch and goes on with the separate kernels)
+enum ST : int { ST_OVERFLOW = 1, ST_LOST = 2, ST_NAN = 4, ST_BOX = 8, ST_BONDS = 16, ST_TIMEOUT = 32 };
 // status bits that end a run with an error (an overflow is healed instead)
 constexpr int ST_FATAL = ST_NAN | ST_LOST | ST_BOX | ST_BONDS;
 
@@ -215,6 +217,7 @@ struct Arena {
   float* ebandf;        // FP32 copy for the mixed kernels
   int4* fxp;            // fixed-point positions (x, y, z, type) for mixed
   double4* pose;        // FP64 force pass: (x, y, z, 1/sqrt(rho)) from the density pass
+  double4* pose2;       // FP64 LJ teams: the second of the two position buffers they gather from
   int4* fxe;            // mixed force pass: (fixed-point x, y, z, bits of float 1/sqrt(rho))
   double2* minv;        // (1/m, 1/sqrt(m))
   double* mass;

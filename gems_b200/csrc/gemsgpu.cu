@@ -21,6 +21,7 @@
 #include "../../include/gemsgpu.h"
 #include "common.cuh"
 #include "kernels.cuh"
+#include "team.cuh"
 #include "lbfgs.cuh"
 #include "neb.cuh"
 
@@ -99,6 +100,25 @@ struct Graph {
   int64_t body_nodes = 0;  // kernels of one conditional rebuild body
 };
 
+// An assignment of systems to teams of CTAs (team.cuh), on the device until
+// another set of systems runs or a shape changes.
+struct TeamPlan {
+  std::string key;         // the systems
+  uint64_t epoch = 0;
+  bool use = false;        // false: the separate kernels serve this set better
+  const void* fn = nullptr;
+  struct Launch {
+    int grid = 0;
+    int cluster = 0;       // resident form: CTAs of a cluster; 0: arena form, a cooperative launch
+    size_t smem = 0;
+    TeamArgs args{};
+  };
+  std::vector<Launch> runs;  // one, or (resident form) one per cluster size, side by side
+  int* buf = nullptr;      // teams, team of each CTA, barrier counters
+  size_t cap = 0;          // ints allocated
+  size_t bar_bytes = 0;
+};
+
 }  // namespace
 
 struct gemsgpu_ctx {
@@ -149,6 +169,12 @@ struct gemsgpu_ctx {
   // for a long time, so a minimisation does not allocate and free its own)
   gg::LbWork lbw{};
   int lbw_m = 0, lbw_scap = 0;
+  // streams of a plan's further launches, and the events that fork and join them
+  std::vector<cudaStream_t> side;
+  std::vector<cudaEvent_t> side_done;
+  cudaEvent_t side_go = nullptr;
+  bool use_team = true;         // whole chunks of small systems in one launch (GEMSGPU_NO_TEAM=1: off)
+  TeamPlan plan;
   double* d_fac = nullptr;      // per-system velocity factors of gemsgpu_retemper
   int d_fac_cap = 0;
 };
@@ -297,6 +323,7 @@ int grow_atoms(gemsgpu_ctx* ctx, int64_t need) {
   CHK(dgrow(ctx, &A.ebandf, keep, nc));
   CHK(dgrow(ctx, &A.fxp, keep, nc));
   CHK(dgrow(ctx, &A.pose, keep, nc));
+  CHK(dgrow(ctx, &A.pose2, keep, nc));
   CHK(dgrow(ctx, &A.fxe, keep, nc));
   CHK(dgrow(ctx, &A.minv, keep, nc));
   CHK(dgrow(ctx, &A.mass, keep, nc));
@@ -977,8 +1004,9 @@ int launch_rebuild(gemsgpu_ctx* ctx, const std::vector<int>& ss, int in_graph = 
   return 0;
 }
 
+// w: a chunk of fused steps opens (velocity Verlet and Ermak systems only)
 int launch_step_a(gemsgpu_ctx* ctx, const std::vector<int>& ss,
-                  cudaGraphConditionalHandle cond = 0, int use_cond = 0) {
+                  cudaGraphConditionalHandle cond = 0, int use_cond = 0, bool w = false) {
   BlockMap ma;
   CHK(get_map(ctx, ss, BLOCK, 0, &ma));
   bool piston = false, lkd = false;
@@ -1000,7 +1028,9 @@ int launch_step_a(gemsgpu_ctx* ctx, const std::vector<int>& ss,
     for (int s : ss)
       if (moving_box(ctx->sys[s].d)) ctx->sys[s].box_live = true;
   }
-  if (use_cond) k_step_a<true><<<ma.nblk, BLOCK, 0, ctx->stream>>>(ctx->A, ma, cond);
+  if (use_cond && w) k_step_a<true, true><<<ma.nblk, BLOCK, 0, ctx->stream>>>(ctx->A, ma, cond);
+  else if (use_cond) k_step_a<true><<<ma.nblk, BLOCK, 0, ctx->stream>>>(ctx->A, ma, cond);
+  else if (w) k_step_a<false, true><<<ma.nblk, BLOCK, 0, ctx->stream>>>(ctx->A, ma, cond);
   else k_step_a<false><<<ma.nblk, BLOCK, 0, ctx->stream>>>(ctx->A, ma, cond);
   ++ctx->launches;
   CU(cudaGetLastError());
@@ -1113,7 +1143,7 @@ int launch_forces_ba(gemsgpu_ctx* ctx, const std::vector<int>& ss, cudaGraphCond
   return 0;
 }
 
-int launch_step_b(gemsgpu_ctx* ctx, const std::vector<int>& ss) {
+int launch_step_b(gemsgpu_ctx* ctx, const std::vector<int>& ss, bool w = false) {
   BlockMap ma;
   CHK(get_map(ctx, ss, BLOCK, 0, &ma));
   bool moves = false, thermo = false, scal = false;
@@ -1123,7 +1153,8 @@ int launch_step_b(gemsgpu_ctx* ctx, const std::vector<int>& ss) {
     thermo |= d.thermo != TH_NONE;
     scal |= d.thermo == TH_SCALVEL || d.thermo == TH_SCALVEL_AFTER;
   }
-  if (moves) k_step_b<true><<<ma.nblk, BLOCK, 0, ctx->stream>>>(ctx->A, ma);
+  if (w) k_step_b<false, true><<<ma.nblk, BLOCK, 0, ctx->stream>>>(ctx->A, ma);
+  else if (moves) k_step_b<true><<<ma.nblk, BLOCK, 0, ctx->stream>>>(ctx->A, ma);
   else k_step_b<false><<<ma.nblk, BLOCK, 0, ctx->stream>>>(ctx->A, ma);
   ++ctx->launches;
   // the thermostats after the integrator's stepb
@@ -1190,33 +1221,335 @@ int estimate_cap(const SysHost& h) {
   return std::max(cap, 16);
 }
 
+// ------------------------------------------------------------- teams
+template <int KIND, int MINB, bool RES>
+const void* team_fn_k(int K) {
+  switch (K) {
+    case 1: return (const void*)k_team<KIND, 1, MINB, RES>;
+    case 2: return (const void*)k_team<KIND, 2, MINB, RES>;
+    case 4: return (const void*)k_team<KIND, 4, MINB, RES>;
+    case 8: return (const void*)k_team<KIND, 8, MINB, RES>;
+    case 16: return (const void*)k_team<KIND, 16, MINB, RES>;
+    default: return (const void*)k_team<KIND, 32, MINB, RES>;
+  }
+}
+
+template <bool RES>
+const void* team_fn(int kind, int K) {
+  switch (kind) {
+    case TK_LJ64: return team_fn_k<TK_LJ64, 2, RES>(K);
+    case TK_LJ32: return team_fn_k<TK_LJ32, 3, RES>(K);
+    case TK_SM64: return team_fn_k<TK_SM64, 2, RES>(K);
+    case TK_SM32: return team_fn_k<TK_SM32, 3, RES>(K);
+    default: return team_fn_k<TK_SM32R, 3, RES>(K);
+  }
+}
+const void* team_fn_tersoff(bool mixed, int K) {
+  if (!mixed) return (const void*)k_team<TK_TS64, 4, 2, false>;
+  return K == 2 ? (const void*)k_team<TK_TS32, 2, 3, false> : (const void*)k_team<TK_TS32, 4, 3, false>;
+}
+
+constexpr int TEAM_MAX_CELLS = 12288;  // a CTA scans the system's cell counts in shared memory
+
+// launch configuration of one launch of a plan
+cudaLaunchConfig_t team_config(const TeamPlan::Launch& R, cudaStream_t st, cudaLaunchAttribute* at) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(R.grid);
+  cfg.blockDim = dim3(BLOCK);
+  cfg.dynamicSmemBytes = R.smem;
+  cfg.stream = st;
+  if (R.cluster > 0) {
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = R.cluster;
+    at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+  } else {
+    at[0].id = cudaLaunchAttributeCooperative;
+    at[0].val.cooperative = 1;
+  }
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  return cfg;
+}
+
+constexpr int TEAM_SMEM = 200 * 1024;  // dynamic shared memory a CTA may ask for
+
+// The cluster sizes of the resident form: a CTA works through r virtual
+// blocks per phase, the fewest that let the device hold every system's
+// cluster at once (systems beyond that queue up), rounded to a power of two;
+// bigger clusters where a system's part would not fit in shared memory.  False
+// if a system fits in none.
+bool team_clusters(gemsgpu_ctx* ctx, const std::vector<int>& ss, const void* fn, int kind, int apb, size_t scratch,
+                   std::vector<int>& C) {
+  int64_t total = 0;
+  for (int s : ss) total += (ctx->sys[s].n + apb - 1) / apb;
+  auto smem = [&](int n, int c) {
+    const int nvb = (n + apb - 1) / apb;
+    return (size_t)res_layout(kind, n, (nvb + c - 1) / c * apb, ctx->A.lcap, (int)scratch).total;
+  };
+  if (cudaFuncSetAttribute(fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess) {
+    cudaGetLastError();
+    return false;
+  }
+  C.assign(ss.size(), 1);
+  for (int r = std::max<int>(1, (int)(total / (4 * ctx->nsm)));; r++) {
+    double sms = 0.0;  // what all clusters together occupy
+    for (size_t k = 0; k < ss.size(); k++) {
+      const int n = ctx->sys[ss[k]].n, nvb = (n + apb - 1) / apb;
+      int c = 1;
+      while (c < 16 && c * r < nvb) c *= 2;
+      if (ss.size() == 1) c = std::min(16, nvb);
+      while (c < 16 && smem(n, c) > (size_t)TEAM_SMEM) c *= 2;
+      if (smem(n, c) > (size_t)TEAM_SMEM) return false;
+      C[k] = c;
+      sms += c * std::max((double)smem(n, c) / (220 * 1024), 1.0 / 3);
+    }
+    if (sms <= 1.5 * ctx->nsm || r >= 32) return true;
+  }
+}
+
+// Assign the systems ss to teams; ctx->plan.use says whether the set runs there.
+int team_plan(gemsgpu_ctx* ctx, const std::vector<int>& ss) {
+  TeamPlan& P = ctx->plan;
+  std::string key;
+  for (int s : ss) key += std::to_string(s) + ",";
+  if (P.key == key && P.epoch == ctx->epoch) return 0;
+  P.key = key;
+  P.epoch = ctx->epoch;
+  P.use = false;
+  if (!ctx->use_team) return 0;
+  const SysHost& h0 = ctx->sys[ss[0]];
+  const int K = h0.d.ff == FF_TERSOFF ? tersoff_lanes(h0) : h0.lanes;
+  const int apb = BLOCK / K;
+  const bool one = h0.ntypes == 1;
+  int maxcell = 0, big = 0;
+  bool w[2] = {false, false};
+  int64_t total = 0, atoms = 0;
+  for (int s : ss) {
+    const SysHost& h = ctx->sys[s];
+    atoms += h.n;
+    const int k = h.d.ff == FF_TERSOFF ? tersoff_lanes(h) : h.lanes;
+    if (h.d.ff == FF_NONE || h.d.ff != h0.d.ff || h.d.prec != h0.d.prec || k != K) return 0;
+    if (h.d.integ != IT_NONE && h.d.integ != IT_VV && h.d.integ != IT_ERMAK && h.d.integ != IT_FIRE) return 0;
+    if (h.d.thermo != TH_NONE || h.d.virial || h.n == 0 || (h.ntypes == 1) != one) return 0;
+    if (h.d.ncell > TEAM_MAX_CELLS) return 0;
+    maxcell = std::max(maxcell, h.d.ncell);
+    if (h.d.use_cells) w[h.d.list_warp == 1] = true;
+    big = std::max(big, h.n);
+    total += (h.n + apb - 1) / apb;
+  }
+  const bool mixed = h0.d.prec == PREC_MIXED;
+  int kind;
+  if (h0.d.ff == FF_LJ) kind = mixed ? TK_LJ32 : TK_LJ64;
+  else if (h0.d.ff == FF_SMATB) kind = !mixed ? TK_SM64 : one ? TK_SM32R : TK_SM32;
+  else kind = mixed ? TK_TS32 : TK_TS64;
+  const bool ts = h0.d.ff == FF_TERSOFF;
+  const size_t tsf = kind == TK_TS64 ? tsf_smem<double, 4>()
+                     : kind == TK_TS32 ? (K == 2 ? tsf_smem<float, 2>() : tsf_smem<float, 4>()) : 0;
+  const size_t scratch = std::max(w[0] || !w[1] ? team_smem(ctx->A.lcap, maxcell, false, tsf) : (size_t)0,
+                                  w[1] ? team_smem(ctx->A.lcap, maxcell, true, tsf) : (size_t)0);
+  P.runs.clear();
+  std::vector<int> all;  // per launch: its teams, then the team of each CTA
+  std::vector<size_t> at_team, at_cta;
+  auto add = [&](const std::vector<Team>& teams, int cluster, size_t smem) {
+    TeamPlan::Launch R;
+    for (const Team& t : teams) R.grid += t.ncta;
+    R.cluster = cluster;
+    R.smem = smem;
+    R.args.nteam = (int)teams.size();
+    R.args.slots = R.grid;
+    at_team.push_back(all.size());
+    for (const Team& t : teams) all.insert(all.end(), {t.cta0, t.ncta, t.sys, t.pad});
+    at_cta.push_back(all.size());
+    for (size_t t = 0; t < teams.size(); t++) all.insert(all.end(), teams[t].ncta, (int)t);
+    while (all.size() % 4) all.push_back(0);
+    P.runs.push_back(R);
+  };
+  // The arena form where it beat the separate kernels and its CTAs fit the
+  // device at once: systems of up to 16000 (LJ) or 32000 atoms, or more atoms
+  // in systems of up to 5000 (us per step, separate -> arena: FP64 LJ 4000
+  // 28.8 -> 17.6, 10976 38.1 -> 32.6, 23328 52.8 -> 58.5; mixed SMA-TB 4000
+  // 26.4 -> 16.9, 23328 35.3 -> 31.4, 70304 50.5 -> 58.6; 16 x 4000 mixed LJ
+  // 80 -> 68; 4 x 10976 FP64 SMA-TB 88 -> 97).  The resident form for smaller
+  // systems, and for batches of small systems that exceed the arena form: one
+  // cluster's few SMs are too little for one system of 2000 atoms (LJ 2048:
+  // 28 -> 42), but 16 clusters of 309 atoms go from 50 to 16, one of 13 from
+  // 20 to 6.
+  const int nmax = h0.d.ff == FF_LJ ? 16000 : 32000;
+  int occ = 0;
+  const void* arena = ts ? team_fn_tersoff(mixed, K) : team_fn<false>(kind, K);
+  const size_t arena_sm = std::max(scratch, tsf);
+  bool arena_ok = arena_sm <= (size_t)TEAM_SMEM && big <= nmax && (atoms <= nmax || big <= 5000);
+  if (arena_ok) {
+    CU(cudaFuncSetAttribute(arena, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)arena_sm));
+    CU(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, arena, BLOCK, arena_sm));
+    arena_ok = total <= (int64_t)occ * ctx->nsm;
+  }
+  std::vector<int> C;
+  const void* fn = ts || big > (arena_ok ? 640 : 2048) ? nullptr : team_fn<true>(kind, K);
+  if (fn && team_clusters(ctx, ss, fn, kind, apb, scratch, C)) {
+    P.fn = fn;
+    std::vector<size_t> order(ss.size());  // the largest first
+    for (size_t k = 0; k < order.size(); k++) order[k] = k;
+    std::stable_sort(order.begin(), order.end(), [&](size_t a, size_t b) {
+      return std::make_pair(C[a], ctx->sys[ss[a]].n) > std::make_pair(C[b], ctx->sys[ss[b]].n);
+    });
+    size_t most = 0;
+    for (size_t k = 0; k < order.size();) {
+      const int c = C[order[k]];
+      std::vector<Team> teams;
+      size_t sm = 0;
+      for (; k < order.size() && C[order[k]] == c; k++) {
+        const int s = ss[order[k]], n = ctx->sys[s].n, nvb = (n + apb - 1) / apb;
+        teams.push_back({(int)teams.size() * c, c, s, 0});
+        sm = std::max(sm, (size_t)res_layout(kind, n, (nvb + c - 1) / c * apb, ctx->A.lcap, (int)scratch).total);
+      }
+      most = std::max(most, sm);
+      add(teams, c, sm);
+    }
+    CU(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most));
+    for (const auto& R : P.runs) {  // a cluster that the device cannot hold is no plan
+      cudaLaunchAttribute at[1];
+      cudaLaunchConfig_t cfg = team_config(R, ctx->stream, at);
+      int nc = 0;
+      if (cudaOccupancyMaxActiveClusters(&nc, fn, &cfg) != cudaSuccess || nc <= 0) {
+        cudaGetLastError();
+        return 0;
+      }
+    }
+    while (ctx->side.size() + 1 < P.runs.size()) {
+      cudaStream_t st;
+      cudaEvent_t ev;
+      CU(cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking));
+      ctx->side.push_back(st);
+      CU(cudaEventCreateWithFlags(&ev, cudaEventDisableTiming));
+      ctx->side_done.push_back(ev);
+    }
+    if (!ctx->side_go) CU(cudaEventCreateWithFlags(&ctx->side_go, cudaEventDisableTiming));
+  } else {
+    if (!arena_ok) return 0;
+    P.fn = arena;
+    std::vector<Team> teams;
+    int ncta = 0;
+    for (int s : ss) {
+      const int c = (ctx->sys[s].n + apb - 1) / apb;
+      teams.push_back({ncta, c, s, 0});
+      ncta += c;
+    }
+    add(teams, 0, arena_sm);
+    CHK(grow_blocks(ctx, 2 * ncta));  // two sets of skin slots (may bump the epoch)
+  }
+  const size_t head = (all.size() + TEAM_BAR - 1) / TEAM_BAR * TEAM_BAR;
+  const size_t bars = (size_t)(ss.size() + 1) * TEAM_BAR;
+  if (P.cap < head + bars) {
+    CHK(dgrow(ctx, &P.buf, 0, 2 * (head + bars)));
+    P.cap = 2 * (head + bars);
+  }
+  CU(cudaMemcpyAsync(P.buf, all.data(), all.size() * sizeof(int), cudaMemcpyHostToDevice, ctx->stream));
+  for (size_t k = 0; k < P.runs.size(); k++) {
+    P.runs[k].args.team = reinterpret_cast<const Team*>(P.buf + at_team[k]);
+    P.runs[k].args.cta_team = P.buf + at_cta[k];
+    P.runs[k].args.bar = reinterpret_cast<unsigned*>(P.buf + head);
+  }
+  P.bar_bytes = bars * sizeof(unsigned);
+  P.epoch = ctx->epoch;
+  P.use = true;
+  return 0;
+}
+
+// the planned launches: `flags` (TF_*), then nsteps steps
+int launch_team(gemsgpu_ctx* ctx, int flags, int nsteps) {
+  TeamPlan& P = ctx->plan;
+  if (!P.runs[0].cluster) CU(cudaMemsetAsync(P.runs[0].args.bar, 0, P.bar_bytes, ctx->stream));
+  const bool several = P.runs.size() > 1;
+  if (several) CU(cudaEventRecord(ctx->side_go, ctx->stream));
+  for (size_t k = 0; k < P.runs.size(); k++) {
+    auto& R = P.runs[k];
+    cudaStream_t st = k == 0 ? ctx->stream : ctx->side[k - 1];
+    if (k > 0) CU(cudaStreamWaitEvent(st, ctx->side_go, 0));
+    R.args.flags = flags;
+    R.args.nsteps = nsteps;
+    void* args[] = {(void*)&ctx->A, (void*)&R.args};
+    cudaLaunchAttribute at[1];
+    const cudaLaunchConfig_t cfg = team_config(R, st, at);
+    CU(cudaLaunchKernelExC(&cfg, P.fn, args));
+    ++ctx->launches;
+    if (k > 0) {
+      CU(cudaEventRecord(ctx->side_done[k - 1], st));
+      CU(cudaStreamWaitEvent(ctx->stream, ctx->side_done[k - 1], 0));
+    }
+  }
+  return 0;
+}
+
+// what a launch has to do before its steps so that every system of ss has
+// its list and forces, or -1 when the systems differ in that
+int team_open(const gemsgpu_ctx* ctx, const std::vector<int>& ss) {
+  int flags = -2;
+  for (int s : ss) {
+    const SysHost& h = ctx->sys[s];
+    const int f = h.first ? TF_REBUILD | TF_FORCE : h.pos_dirty ? TF_SKIN | TF_FORCE : h.has_forces ? 0 : -1;
+    if (flags == -2) flags = f;
+    if (f != flags) return -1;
+  }
+  return flags;
+}
+
+// lists of the neighbour capacity a first build of ss is expected to need
+int ensure_list(gemsgpu_ctx* ctx, const std::vector<int>& ss) {
+  int need = 0;
+  for (int s : ss) need = std::max(need, estimate_cap(ctx->sys[s]));
+  if (ctx->A.lcap < need) CHK(grow_list(ctx, need));
+  return 0;
+}
+
 // interact (src/Interaction.f90:135-241) for a set of systems, host-driven:
 // rebuild if flagged (heal overflow by growing the list), then forces.
+void settled(gemsgpu_ctx* ctx, const std::vector<int>& ss);
+
 int interact_group(gemsgpu_ctx* ctx, const std::vector<int>& ss, bool sync_check) {
-  std::vector<int> first, dirty;
-  int need = 0;
-  for (int s : ss) {
-    SysHost& h = ctx->sys[s];
-    if (h.first) first.push_back(s);
-    else if (h.pos_dirty) dirty.push_back(s);
-    need = std::max(need, estimate_cap(h));
+  CHK(ensure_list(ctx, ss));
+  bool built = false;  // h_st holds the states after a list update
+  const int open = sync_check ? team_open(ctx, ss) : -1;
+  if (open > 0) {
+    // small systems: lists and forces in one launch
+    CHK(team_plan(ctx, ss));
+    if (ctx->plan.use && ctx->plan.runs[0].cluster) {
+      CHK(clear_status(ctx, ss));
+      CHK(launch_team(ctx, open, 0));
+      CHK(read_states(ctx));
+      bool over = false;
+      for (int s : ss) over |= (ctx->h_st[s].status & ST_OVERFLOW) != 0;
+      if (!over) {
+        for (int s : ss) CHK(status_error(ctx, s, ctx->h_st[s].status));
+        settled(ctx, ss);
+        return 0;
+      }
+      built = true;  // a list overflowed: grown and built again below
+    }
   }
-  if (ctx->A.lcap < need) CHK(grow_list(ctx, need));
-  CHK(clear_status(ctx, ss));
-  if (!first.empty()) {
-    const int* sa;
-    CHK(sys_array(ctx, first, &sa));
-    k_force_rebuild<<<((int)first.size() + 255) / 256, 256, 0, ctx->stream>>>(ctx->A, sa,
-                                                                                 (int)first.size()); ++ctx->launches;
+  if (!built) {
+    std::vector<int> first, dirty;
+    for (int s : ss) {
+      SysHost& h = ctx->sys[s];
+      if (h.first) first.push_back(s);
+      else if (h.pos_dirty) dirty.push_back(s);
+    }
+    CHK(clear_status(ctx, ss));
+    if (!first.empty()) {
+      const int* sa;
+      CHK(sys_array(ctx, first, &sa));
+      k_force_rebuild<<<((int)first.size() + 255) / 256, 256, 0, ctx->stream>>>(ctx->A, sa,
+                                                                                   (int)first.size()); ++ctx->launches;
+    }
+    if (!dirty.empty()) {
+      BlockMap m;
+      CHK(get_map(ctx, dirty, BLOCK, 0, &m));
+      k_skin<<<m.nblk, BLOCK, 0, ctx->stream>>>(ctx->A, m); ++ctx->launches;
+    }
+    CHK(launch_rebuild(ctx, ss));
+    if (sync_check) CHK(read_states(ctx));
   }
-  if (!dirty.empty()) {
-    BlockMap m;
-    CHK(get_map(ctx, dirty, BLOCK, 0, &m));
-    k_skin<<<m.nblk, BLOCK, 0, ctx->stream>>>(ctx->A, m); ++ctx->launches;
-  }
-  CHK(launch_rebuild(ctx, ss));
   if (sync_check) {
-    CHK(read_states(ctx));
     int grow = 0;
     for (int s : ss) {
       const SysState& st = ctx->h_st[s];
@@ -1281,25 +1614,25 @@ int record_steps(gemsgpu_ctx* ctx, const std::vector<int>& ss, int n) {
   if (ss.size() == 1 && can_fuse_forces(ctx, ss)) {
     // step_a, then per step: rebuild chain, density pass, force pass with
     // step_b + the next step_a; the last step closes with its own step_b
-    CHK(launch_step_a(ctx, ss));
+    CHK(launch_step_a(ctx, ss, 0, 0, true));
     for (int k = 0; k < n; k++) {
       CHK(launch_rebuild(ctx, ss));
       if (k < n - 1) {
         CHK(launch_forces_ba(ctx, ss));
       } else {
         CHK(launch_forces(ctx, ss));
-        CHK(launch_step_b(ctx, ss));
+        CHK(launch_step_b(ctx, ss, true));
       }
     }
     return 0;
   }
   const bool fuse = can_fuse_steps(ctx, ss);
   for (int k = 0; k < n; k++) {
-    if (k == 0 || !fuse) CHK(launch_step_a(ctx, ss));
+    if (k == 0 || !fuse) CHK(launch_step_a(ctx, ss, 0, 0, fuse));
     else CHK(launch_step_ba(ctx, ss));
     CHK(launch_rebuild(ctx, ss));
     CHK(launch_forces(ctx, ss));
-    if (!fuse || k == n - 1) CHK(launch_step_b(ctx, ss));
+    if (!fuse || k == n - 1) CHK(launch_step_b(ctx, ss, fuse));
   }
   return 0;
 }
@@ -1336,7 +1669,7 @@ struct CondArg {
 };
 
 int cap_step_a(gemsgpu_ctx* ctx, const std::vector<int>& ss, void* arg) {
-  return launch_step_a(ctx, ss, ((CondArg*)arg)->h, 1);
+  return launch_step_a(ctx, ss, ((CondArg*)arg)->h, 1, can_fuse_steps(ctx, ss));
 }
 int cap_step_ba(gemsgpu_ctx* ctx, const std::vector<int>& ss, void* arg) {
   return launch_step_ba(ctx, ss, ((CondArg*)arg)->h, 1);
@@ -1350,7 +1683,7 @@ int cap_rebuild(gemsgpu_ctx* ctx, const std::vector<int>& ss, void*) {
 }
 int cap_forces_b(gemsgpu_ctx* ctx, const std::vector<int>& ss, void*) {
   CHK(launch_forces(ctx, ss));
-  return launch_step_b(ctx, ss);
+  return launch_step_b(ctx, ss, can_fuse_steps(ctx, ss));
 }
 int cap_forces(gemsgpu_ctx* ctx, const std::vector<int>& ss, void*) {
   return launch_forces(ctx, ss);
@@ -1603,53 +1936,109 @@ int snapshot(gemsgpu_ctx* ctx, bool restore) {
   return 0;
 }
 
-constexpr int CHUNK = 50;
+constexpr int CHUNK = 50;        // steps of a captured graph
+constexpr int TEAM_CHUNK = 200;  // steps of a team launch
+
+int refresh_fx(gemsgpu_ctx* ctx, const std::vector<int>& ss) {
+  BlockMap m;
+  CHK(get_map(ctx, ss, BLOCK, 0, &m));
+  k_refresh_fx<<<m.nblk, BLOCK, 0, ctx->stream>>>(ctx->A, m); ++ctx->launches;
+  return 0;
+}
+
+void settled(gemsgpu_ctx* ctx, const std::vector<int>& ss) {
+  for (int s : ss) {
+    SysHost& h = ctx->sys[s];
+    h.first = false;
+    h.pos_dirty = false;
+    h.has_forces = true;
+  }
+}
+
+// Run one chunk of k steps of ss, in teams (opened by `open`, TF_* flags) or
+// as a captured graph, and check the states.  A chunk that overflowed a list
+// is undone, the list grown and *redo set; so is one whose team barrier gave
+// up, after which the separate kernels run.
+int run_chunk(gemsgpu_ctx* ctx, const std::vector<int>& ss, bool team, int open, int k, bool* redo) {
+  *redo = false;
+  CHK(snapshot(ctx, false));
+  CHK(clear_status(ctx, ss));
+  if (team) CHK(launch_team(ctx, open, k));
+  else CHK(launch_graph(ctx, ss, k));
+  CHK(read_states(ctx));
+  int grow = 0, bad = 0, bads = -1;
+  bool late = false;
+  for (int s : ss) {
+    int st = ctx->h_st[s].status;
+    if (st & ST_OVERFLOW) grow = std::max(grow, ctx->h_st[s].maxnn);
+    if (st & ST_FATAL) { bad = st; bads = s; }
+    late |= (st & ST_TIMEOUT) != 0;
+  }
+  if (late) {
+    CHK(snapshot(ctx, true));
+    CHK(refresh_fx(ctx, ss));
+    CU(cudaMemsetAsync(ctx->A.cell_count, 0, ctx->ccap * sizeof(int), ctx->stream));  // left mid-rebuild
+    ctx->use_team = false;
+    invalidate(ctx);
+    for (int s : ss) ctx->sys[s].first = true;
+    CHK(interact_group(ctx, ss, true));
+    *redo = true;
+    return 0;
+  }
+  if (bad) {
+    if (open) {  // refused at the opening evaluation or after it: nothing has moved
+      CHK(snapshot(ctx, true));
+      CHK(refresh_fx(ctx, ss));
+    }
+    return status_error(ctx, bads, bad);
+  }
+  if (grow == 0) {
+    settled(ctx, ss);
+  } else {
+    *redo = true;
+    CHK(snapshot(ctx, true));
+    CHK(refresh_fx(ctx, ss));  // the fixed-point copies were left at the undone chunk's positions
+    if (open) return interact_group(ctx, ss, true);
+    CHK(grow_list(ctx, grow + grow / 4 + 8));
+    const int* sa;
+    CHK(sys_array(ctx, ss, &sa));
+    k_force_rebuild<<<((int)ss.size() + 255) / 256, 256, 0, ctx->stream>>>(ctx->A, sa, (int)ss.size()); ++ctx->launches;
+    CHK(clear_status(ctx, ss));
+    CHK(launch_rebuild(ctx, ss));
+    CHK(launch_forces(ctx, ss));
+  }
+  return 0;
+}
 
 // dinamic (src/Programs.f90:114-167) for a set of systems, device-resident:
-// chunks of CHUNK captured steps; after each chunk the states are checked,
-// and a chunk that overflowed a list is undone, the list grown and redone.
+// chunks of steps, the states checked after each
 int md_group(gemsgpu_ctx* ctx, const std::vector<int>& ss, int nsteps) {
   for (int s : ss) {
     const SysHost& h = ctx->sys[s];
     if (h.d.integ == IT_NONE) return fail(ctx, GEMSGPU_ERR_STATE, "system %d has no integrator", s);
   }
-  bool need_first = false;
-  for (int s : ss) need_first |= ctx->sys[s].first || ctx->sys[s].pos_dirty || !ctx->sys[s].has_forces;
-  if (need_first) CHK(interact_group(ctx, ss, true));
+  CHK(ensure_list(ctx, ss));
+  // a team launch takes the opening interact along
+  CHK(team_plan(ctx, ss));
+  int open = ctx->plan.use && nsteps > 0 ? team_open(ctx, ss) : -1;
+  if (open < 0) {
+    bool need_first = false;
+    for (int s : ss) need_first |= ctx->sys[s].first || ctx->sys[s].pos_dirty || !ctx->sys[s].has_forces;
+    if (need_first) CHK(interact_group(ctx, ss, true));
+    open = 0;
+  }
   int done = 0;
   int retries = 0;
   while (done < nsteps) {
-    int k = std::min(CHUNK, nsteps - done);
-    CHK(snapshot(ctx, false));
-    CHK(clear_status(ctx, ss));
-    CHK(launch_graph(ctx, ss, k));
-    CHK(read_states(ctx));
-    int grow = 0, bad = 0, bads = -1;
-    for (int s : ss) {
-      int st = ctx->h_st[s].status;
-      if (st & ST_OVERFLOW) grow = std::max(grow, ctx->h_st[s].maxnn);
-      if (st & ST_FATAL) { bad = st; bads = s; }
-    }
-    if (bad) return status_error(ctx, bads, bad);
-    if (grow > 0) {
-      if (++retries > 4) return fail(ctx, GEMSGPU_ERR_OVERFLOW, "neighbour list keeps overflowing");
-      CHK(snapshot(ctx, true));
-      {
-        // the fixed-point copies were left at the undone chunk's positions
-        BlockMap mr;
-        CHK(get_map(ctx, ss, BLOCK, 0, &mr));
-        k_refresh_fx<<<mr.nblk, BLOCK, 0, ctx->stream>>>(ctx->A, mr); ++ctx->launches;
-      }
-      CHK(grow_list(ctx, grow + grow / 4 + 8));
-      const int* sa;
-      CHK(sys_array(ctx, ss, &sa));
-      k_force_rebuild<<<((int)ss.size() + 255) / 256, 256, 0, ctx->stream>>>(ctx->A, sa, (int)ss.size()); ++ctx->launches;
-      CHK(clear_status(ctx, ss));
-      CHK(launch_rebuild(ctx, ss));
-      CHK(launch_forces(ctx, ss));
-      continue;
-    }
-    done += k;
+    CHK(team_plan(ctx, ss));  // again after a list grew
+    const bool team = ctx->plan.use;
+    if (!team && open) CHK(interact_group(ctx, ss, true));
+    const int k = std::min(team ? TEAM_CHUNK : CHUNK, nsteps - done);
+    bool redo;
+    CHK(run_chunk(ctx, ss, team, team ? open : 0, k, &redo));
+    open = 0;
+    if (!redo) done += k;
+    else if (++retries > 4) return fail(ctx, GEMSGPU_ERR_OVERFLOW, "neighbour list keeps overflowing");
   }
   return 0;
 }
@@ -1995,6 +2384,7 @@ int gemsgpu_create(int device, int64_t max_atoms, int max_systems, gemsgpu_ctx**
   // profilers cannot replay kernels of graphs with conditional nodes:
   // GEMSGPU_NO_COND=1 captures plain steps (rebuild kernels exit early)
   if (const char* e = getenv("GEMSGPU_NO_COND")) ctx->use_cond = !(e[0] == '1');
+  if (const char* e = getenv("GEMSGPU_NO_TEAM")) ctx->use_team = !(e[0] == '1');
   if (const char* e = getenv("GEMSGPU_NO_FUSED_FORCES")) ctx->fuse_forces = !(e[0] == '1');
   int rc = 0;
   do {
@@ -2033,18 +2423,21 @@ int gemsgpu_destroy(gemsgpu_ctx* ctx) {
   drop_maps(ctx);
   Arena& A = ctx->A;
   void* ptrs[] = {A.pos, A.pos_old, A.vel, A.acel, A.force, A.vel_v, A.acel2, A.acel3, A.acel4, A.epot, A.band, A.eband,
-                  A.ebandf, A.fxp, A.pose, A.fxe, A.minv, A.mass, A.type, A.nn, A.hnn, A.ncut, A.list, A.flist, A.cell_of, A.slot,
+                  A.ebandf, A.fxp, A.pose, A.pose2, A.fxe, A.minv, A.mass, A.type, A.nn, A.hnn, A.ncut, A.list, A.flist, A.cell_of, A.slot,
                   A.cell_count, A.cell_n, A.cell_loc, A.cell_start, A.chunk_sum, A.cell_atoms,
                   A.cell_pos, A.rslot, A.tidx, A.tsmask, A.tsfb, A.tsfb32,
                   A.ext_normals, A.blk_top2, A.blk_red, A.sys, A.st, A.prm, A.any_rebuild, A.body_runs,
                   ctx->d_red, ctx->snap, ctx->snap_st, ctx->snap_sys, ctx->d_sys,
                   ctx->lbw.x0, ctx->lbw.g, ctx->lbw.gold, ctx->lbw.d, ctx->lbw.S, ctx->lbw.Y, ctx->lbw.st,
-                  ctx->d_fac};
+                  ctx->d_fac, ctx->plan.buf};
   for (void* p : ptrs)
     if (p) cudaFree(p);
   if (ctx->h_red) cudaFreeHost(ctx->h_red);
   if (ctx->h_st) cudaFreeHost(ctx->h_st);
   if (ctx->stage) cudaFree(ctx->stage);
+  for (auto st : ctx->side) cudaStreamDestroy(st);
+  for (auto ev : ctx->side_done) cudaEventDestroy(ev);
+  if (ctx->side_go) cudaEventDestroy(ctx->side_go);
   if (ctx->stream) cudaStreamDestroy(ctx->stream);
   delete ctx;
   return 0;
@@ -3113,7 +3506,23 @@ int gemsgpu_batch_fire(gemsgpu_ctx* ctx, const int* sys, int nsys, double fmax, 
     atoms += h.n;
     cells += h.d.use_cells ? h.d.ncell : 0;
   }
-  if (uniform) {
+  CHK(team_plan(ctx, ss));
+  if (uniform && ctx->plan.use) {
+    // small systems: chunks in teams, the unconverged systems each time
+    int retries = 0;
+    for (;;) {
+      CHK(read_states(ctx));
+      std::vector<int> act;
+      for (int s : ss)
+        if (!ctx->h_st[s].fire_done) act.push_back(s);
+      if (act.empty() || total >= maxit) break;
+      CHK(team_plan(ctx, act));
+      bool redo;
+      CHK(run_chunk(ctx, act, ctx->plan.use, 0, CHUNK, &redo));
+      if (!redo) total += CHUNK;
+      else if (++retries > 4) return fail(ctx, GEMSGPU_ERR_OVERFLOW, "neighbour list keeps overflowing");
+    }
+  } else if (uniform) {
     // converged systems leave the pool's active set between chunks
     const SysHost& h0 = ctx->sys[ss[0]];
     gemsgpu_pool* P = nullptr;
@@ -3316,13 +3725,20 @@ static int autotune_set(gemsgpu_ctx* ctx, const std::vector<int>& ss, int reps, 
       ctx->sys[s].lanes = c.first;
       ctx->sys[s].variant = c.second;
     }
-    CHK(launch_forces(ctx, ss));  // warm-up (and map creation)
+    // small systems step in teams: their evaluation is timed in the form that
+    // will run it
+    invalidate(ctx);
+    CHK(team_plan(ctx, ss));
+    const bool team = ctx->plan.use;
+    auto once = [&]() -> int { return team ? launch_team(ctx, TF_FORCE, 0) : launch_forces(ctx, ss); };
+    CHK(once());  // warm-up (and map creation)
     CU(cudaEventRecord(e0, ctx->stream));
-    for (int r = 0; r < reps; r++) CHK(launch_forces(ctx, ss));
+    for (int r = 0; r < reps; r++) CHK(once());
     CU(cudaEventRecord(e1, ctx->stream));
     CU(cudaEventSynchronize(e1));
     float ms;
     CU(cudaEventElapsedTime(&ms, e0, e1));
+    if (!team) ms += 0.012f * reps;  // the step's other launches, which a team does not have
     if (ms / reps < best) {
       best = ms / reps;
       pick = c;

@@ -63,6 +63,13 @@ __device__ __forceinline__ void bm_pair(uint32_t a, uint32_t b, double& n1, doub
   n2 = (double)(rr * sn);
 }
 
+// the pair of coordinate c of normals6
+__device__ __forceinline__ void normals_c(uint32_t atom, uint64_t step, uint64_t seed, int c, double& r0, double& r1) {
+  const uint2 key = make_uint2((uint32_t)seed, (uint32_t)(seed >> 32));
+  const uint4 q = philox10(make_uint4(atom, (uint32_t)step, (uint32_t)(step >> 32), c == 2 ? 1u : 0u), key);
+  bm_pair(c == 1 ? q.z : q.x, c == 1 ? q.w : q.y, r0, r1);
+}
+
 // six standard normals for (atom, step) from two Philox blocks
 __device__ __forceinline__ void normals6(uint32_t atom, uint64_t step, uint64_t seed, double r[6]) {
   const uint2 key = make_uint2((uint32_t)seed, (uint32_t)(seed >> 32));
@@ -145,15 +152,94 @@ __device__ __forceinline__ double rd_exact(const SysDev& S, double4 xi, double4 
   return __dadd_rn(__dadd_rn(__dmul_rn(v0, v0), __dmul_rn(v1, v1)), __dmul_rn(v2, v2));
 }
 
-// minimum-image pair vector in FP64 for the FP64 force kernels
-__device__ __forceinline__ void vd_fp64(const SysDev& S, double4 xi, double4 xj,
-                                        double& v0, double& v1, double& v2) {
-  v0 = xj.x - xi.x;
-  v1 = xj.y - xi.y;
-  v2 = xj.z - xi.z;
-  if (S.pbc[0]) v0 = v0 - S.L[0] * round(v0 * S.invL[0]);
-  if (S.pbc[1]) v1 = v1 - S.L[1] * round(v1 * S.invL[1]);
-  if (S.pbc[2]) v2 = v2 - S.L[2] * round(v2 * S.invL[2]);
+// minimum-image pair vector in FP64 for the FP64 force kernels.  A component
+// below 0.4999 L in magnitude has the image number round(v / L) = 0, which an
+// integer comparison of high words decides; only pairs across a box face (or
+// of atoms outside the box) take the rounding, so few warps pay for it.
+struct ImgTest {
+  int h[3];  // high words of 0.4999 L (open dims: no component reaches it)
+};
+__device__ __forceinline__ ImgTest img_test(const SysDev& S) {
+  ImgTest t;
+#pragma unroll
+  for (int d = 0; d < 3; d++) t.h[d] = S.pbc[d] ? __double2hiint(0.4999 * S.L[d]) : 0x7fffffff;
+  return t;
+}
+template <int N>
+__device__ __forceinline__ void vd_fp64(const SysDev& S, const ImgTest& t, double4 xi, const double4 (&xj)[N],
+                                        double (&v)[N][3]) {
+  bool far = false;
+#pragma unroll
+  for (int u = 0; u < N; u++) {
+    v[u][0] = xj[u].x - xi.x;
+    v[u][1] = xj[u].y - xi.y;
+    v[u][2] = xj[u].z - xi.z;
+#pragma unroll
+    for (int d = 0; d < 3; d++) far |= (__double2hiint(v[u][d]) & 0x7fffffff) >= t.h[d];
+  }
+  if (far) {
+#pragma unroll
+    for (int u = 0; u < N; u++)
+#pragma unroll
+      for (int d = 0; d < 3; d++)
+        if (S.pbc[d]) v[u][d] = v[u][d] - S.L[d] * round(v[u][d] * S.invL[d]);
+  }
+}
+
+// 1/a for normal positive a: the hardware's coarse estimate and one third-order
+// step y (1 + e + e^2), e = 1 - a y (the truncated geometric series of
+// 1 / (1 - e)).  The FP64 pipe runs these in a third of the instructions of
+// the exact division.
+__device__ __forceinline__ double rcp_pos(double a) {
+  double y;
+  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(a));
+  const double e = fma(-a, y, 1.0);
+  return fma(y, fma(e, e, e), y);
+}
+
+// r = sqrt(a) and 1/r: the hardware's coarse estimate of 1/sqrt(a), one step
+// of Halley's iteration, and a Newton step for r.  Branch-free, so the pairs
+// of a group interleave; zero and tiny a (coincident atoms) give r ~ 0 and
+// 1/r = infinity.
+__device__ __forceinline__ double sqrt_pos(double a, double& rinv) {
+  const bool tiny = __double2hiint(a) < 0x00200000;
+  a = tiny ? 1e-300 : a;
+  double y;
+  asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(a));
+  const double e = fma(-a * y, y, 1.0);
+  y = fma(y * e, fma(0.375, e, 0.5), y);
+  const double r = a * y;
+  rinv = tiny ? __hiloint2double(0x7ff00000, 0) : y;
+  return fma(fma(-r, r, a), 0.5 * y, r);
+}
+
+// exp(x) for |x| < EXP_MID: x = n ln 2 + f with |f| <= ln(2)/2, the Taylor
+// polynomial of exp(f) to degree 13 (remainder below 5e-18), and n added to
+// the exponent.  No branches (the library's exp has one for its special
+// cases), so the exponentials of a group of pairs interleave: the FP64 pair
+// kernels are bound by the latency of these chains, not by the FP64 rate.
+constexpr double EXP_MID = 600.0;
+__device__ __forceinline__ double exp_mid(double x) {
+  const double big = 6755399441055744.0;  // 1.5 2^52: the sum's low word is round(x / ln 2)
+  const double t = fma(x, 1.4426950408889634074, big);
+  const double n = t - big;
+  double f = fma(n, -0.69314718055994530942, x);
+  f = fma(n, -2.3190468138462995584e-17, f);
+  double p = 1.0 / 6227020800.0;
+  p = fma(p, f, 1.0 / 479001600.0);
+  p = fma(p, f, 1.0 / 39916800.0);
+  p = fma(p, f, 1.0 / 3628800.0);
+  p = fma(p, f, 1.0 / 362880.0);
+  p = fma(p, f, 1.0 / 40320.0);
+  p = fma(p, f, 1.0 / 5040.0);
+  p = fma(p, f, 1.0 / 720.0);
+  p = fma(p, f, 1.0 / 120.0);
+  p = fma(p, f, 1.0 / 24.0);
+  p = fma(p, f, 1.0 / 6.0);
+  p = fma(p, f, 0.5);
+  p = fma(p, f, 1.0);
+  p = fma(p, f, 1.0);
+  return __hiloint2double(__double2hiint(p) + (__double2loint(t) << 20), __double2loint(p));
 }
 
 // fixed-point coordinates for the mixed kernels.  Periodic dims map [0,L)
@@ -173,14 +259,17 @@ __device__ __forceinline__ int fx_coord(const SysDev& S, int d, double x, int& b
   return (int)t;
 }
 
-__device__ __forceinline__ void write_fx(const Arena& A, const SysDev& S, int i,
-                                         double4 p, int ti, int& bad) {
+__device__ __forceinline__ int4 fx_record(const SysDev& S, double4 p, int ti, int& bad) {
   int4 q;
   q.x = fx_coord(S, 0, p.x, bad);
   q.y = fx_coord(S, 1, p.y, bad);
   q.z = fx_coord(S, 2, p.z, bad);
   q.w = ti;
-  A.fxp[i] = q;
+  return q;
+}
+__device__ __forceinline__ void write_fx(int4* fxp, const SysDev& S, int i,
+                                         double4 p, int ti, int& bad) {
+  fxp[i] = fx_record(S, p, ti, bad);
 }
 
 // squared displacement since the last rebuild.  Reference mode (skin_mic=0)
@@ -188,6 +277,11 @@ __device__ __forceinline__ void write_fx(const Arena& A, const SysDev& S, int i,
 // wrapped by do_pbc counts as having moved a box length and forces a rebuild;
 // skin_mic=1 takes the minimum image, which moves no list decision for atoms
 // that did not move, only skips those spurious rebuilds.
+__device__ __forceinline__ double disp_c(const SysDev& S, int c, double x, double q) {  // coordinate c, squared
+  double v = __dsub_rn(x, q);
+  if (S.skin_mic && S.pbc[c]) v = __dsub_rn(v, __dmul_rn(S.L[c], round(__dmul_rn(v, S.invL[c]))));
+  return __dmul_rn(v, v);
+}
 __device__ __forceinline__ double disp2(const SysDev& S, double4 x, double4 q) {
   double v0 = __dsub_rn(x.x, q.x), v1 = __dsub_rn(x.y, q.y), v2 = __dsub_rn(x.z, q.z);
   if (S.skin_mic) {
@@ -307,21 +401,15 @@ __global__ void k_refresh_fx(Arena A, BlockMap M) {
   if (i >= M.end[blockIdx.x]) return;
   const SysDev& S = A.sys[s];
   int bad = 0;
-  write_fx(A, S, i, A.pos[i], A.type[i], bad);
+  write_fx(A.fxp, S, i, A.pos[i], A.type[i], bad);
   if (bad) atomicOr(&A.st[s].status, ST_LOST);
 }
 
 // ------------------------------------------------------------------ binning
 // sort_in_cells (src/Neighbour.F90:927-989) as a counting sort:
 // k_bin (histogram) -> k_scan1/k_scan2 (prefix) -> k_scatter -> k_sort_cells
-__global__ void k_bin(Arena A, BlockMap M) {
-  int s = blk_sys(M);
-  if (s < 0) return;  // padding block of a fixed-capacity map
-  const SysDev& S = A.sys[s];
-  if (!A.st[s].rebuild || !S.use_cells) return;
-  int i = M.first[blockIdx.x] + threadIdx.x;
-  if (i >= M.end[blockIdx.x]) return;
-  double4 p = A.pos[i];
+// the grid cell of a position
+__device__ __forceinline__ int atom_cell(const Arena& A, int s, const SysDev& S, double4 p) {
   int c0 = (int)__dmul_rn(p.x, S.inv_cell[0]);
   int c1 = (int)__dmul_rn(p.y, S.inv_cell[1]);
   int c2 = (int)__dmul_rn(p.z, S.inv_cell[2]);
@@ -332,7 +420,17 @@ __global__ void k_bin(Arena A, BlockMap M) {
   if (c1 < 0 || c1 >= S.nc[1]) { lost = true; c1 = c1 < 0 ? 0 : S.nc[1] - 1; }
   if (c2 < 0 || c2 >= S.nc[2]) { lost = true; c2 = c2 < 0 ? 0 : S.nc[2] - 1; }
   if (lost || !(p.x == p.x && p.y == p.y && p.z == p.z)) atomicOr(&A.st[s].status, ST_LOST);
-  int cid = S.cell_off + c0 + S.nc[0] * (c1 + S.nc[1] * c2);
+  return S.cell_off + c0 + S.nc[0] * (c1 + S.nc[1] * c2);
+}
+
+__global__ void k_bin(Arena A, BlockMap M) {
+  int s = blk_sys(M);
+  if (s < 0) return;  // padding block of a fixed-capacity map
+  const SysDev& S = A.sys[s];
+  if (!A.st[s].rebuild || !S.use_cells) return;
+  int i = M.first[blockIdx.x] + threadIdx.x;
+  if (i >= M.end[blockIdx.x]) return;
+  const int cid = atom_cell(A, s, S, A.pos[i]);
   A.cell_of[i] = cid;
   A.slot[i] = atomicAdd(&A.cell_count[cid], 1);
 }
@@ -440,52 +538,56 @@ __device__ __forceinline__ bool rebuild_block(const Arena& A, const BlockMap& M,
   return s >= 0 && A.st[s].rebuild && (A.sys[s].use_cells != 0) == cells;
 }
 
+// one warp orders the n atoms of the cell whose atoms start at `start`
+__device__ __forceinline__ void sort_cell(const Arena& A, int start, int n, int ln) {
+  int* a = A.cell_atoms + start;
+  if (n <= 64) {
+    int v0 = ln < n ? a[ln] : -1;
+    int v1 = ln + 32 < n ? a[ln + 32] : -1;
+    int r0 = 0, r1 = 0;
+    // rank = entries greater than mine; empty slots (-1) are greater than none
+    for (int k = 0; k < min(n, 32); k++) {
+      const int w0 = __shfl_sync(0xffffffffu, v0, k);
+      r0 += w0 > v0;
+      r1 += w0 > v1;
+    }
+    for (int k = 0; k < n - 32; k++) {
+      const int w1 = __shfl_sync(0xffffffffu, v1, k);
+      r0 += w1 > v0;
+      r1 += w1 > v1;
+    }
+    __syncwarp();
+    // each lane places its own atoms (id and position) at their ranks
+    if (ln < n) {
+      a[r0] = v0;
+      A.cell_pos[start + r0] = A.pos[v0];
+    }
+    if (ln + 32 < n) {
+      a[r1] = v1;
+      A.cell_pos[start + r1] = A.pos[v1];
+    }
+  } else if (ln == 0) {
+    for (int x = 1; x < n; x++) {
+      int v = a[x];
+      int y = x - 1;
+      while (y >= 0 && a[y] < v) {
+        a[y + 1] = a[y];
+        y--;
+      }
+      a[y + 1] = v;
+    }
+    for (int x = 0; x < n; x++) A.cell_pos[start + x] = A.pos[a[x]];  // the lane's own writes
+  }
+}
+
 __global__ void k_sort_cells(Arena A, BlockMap C) {
   rebuild_items(C.nblk, [&](int b) { return rebuild_block(A, C, b, true); }, [&](int b) {
     const int warp = threadIdx.x >> 5, ln = threadIdx.x & 31;
     const int first = C.first[b], end = C.end[b];
     for (int c = first + warp; c < end; c += BLOCK / 32) {  // C: 8 cells per block
-      int start = A.chunk_sum[c >> 8] + A.cell_loc[c];
-      int n = A.cell_n[c];
+      const int start = A.chunk_sum[c >> 8] + A.cell_loc[c];
       if (ln == 0) A.cell_start[c] = start;
-      int* a = A.cell_atoms + start;
-      if (n <= 64) {
-        int v0 = ln < n ? a[ln] : -1;
-        int v1 = ln + 32 < n ? a[ln + 32] : -1;
-        int r0 = 0, r1 = 0;
-        // rank = entries greater than mine; empty slots (-1) are greater than none
-        for (int k = 0; k < min(n, 32); k++) {
-          const int w0 = __shfl_sync(0xffffffffu, v0, k);
-          r0 += w0 > v0;
-          r1 += w0 > v1;
-        }
-        for (int k = 0; k < n - 32; k++) {
-          const int w1 = __shfl_sync(0xffffffffu, v1, k);
-          r0 += w1 > v0;
-          r1 += w1 > v1;
-        }
-        __syncwarp();
-        // each lane places its own atoms (id and position) at their ranks
-        if (ln < n) {
-          a[r0] = v0;
-          A.cell_pos[start + r0] = A.pos[v0];
-        }
-        if (ln + 32 < n) {
-          a[r1] = v1;
-          A.cell_pos[start + r1] = A.pos[v1];
-        }
-      } else if (ln == 0) {
-        for (int x = 1; x < n; x++) {
-          int v = a[x];
-          int y = x - 1;
-          while (y >= 0 && a[y] < v) {
-            a[y + 1] = a[y];
-            y--;
-          }
-          a[y + 1] = v;
-        }
-        for (int x = 0; x < n; x++) A.cell_pos[start + x] = A.pos[a[x]];  // the lane's own writes
-      }
+      sort_cell(A, start, A.cell_n[c], ln);
     }
     });
 }
@@ -580,14 +682,24 @@ __device__ __forceinline__ void list_force_order(const Arena& A, const SysDev& S
   }
 }
 
-// the flist entries an atom's force loop must visit this step
-__device__ __forceinline__ int live_entries(const Arena& A, const SysDev& S, const SysState& st, int i, int nn) {
-  if (!(S.skin > 0.0) || !S.use_cells) return nn;  // O(N^2) lists are not grouped by band
+// which of an atom's skip counts bounds its force loop this step: the first
+// threshold k with k skin/7 >= D (8: none, every entry; O(N^2) lists are not
+// grouped by band)
+__device__ __forceinline__ int live_band(const SysDev& S, const SysState& st) {
+  if (!(S.skin > 0.0) || !S.use_cells) return 8;
   const double q = st.dmax * 7.0 / S.skin;
-  if (!(q <= 7.0)) return nn;
-  const int k = (int)ceil(q);
-  const unsigned w = __ldg(reinterpret_cast<const unsigned*>(A.ncut + i) + (k >> 1));
-  return min(nn, (int)((k & 1) ? (w >> 16) : (w & 0xffffu)));
+  if (!(q <= 7.0)) return 8;
+  return (int)ceil(q);
+}
+
+// the flist entries an atom's force loop must visit this step (NC: the lists
+// do not change during the kernel, so they are read through the read-only path)
+template <bool NC = true>
+__device__ __forceinline__ int live_entries(const Arena& A, int lk, int i, int nn) {
+  if (lk > 7) return nn;
+  const unsigned* p = reinterpret_cast<const unsigned*>(A.ncut + i) + (lk >> 1);
+  const unsigned w = NC ? __ldg(p) : *p;
+  return min(nn, (int)((lk & 1) ? (w >> 16) : (w & 0xffffu)));
 }
 
 // A warp's staged row of atom i (m accepted candidates in the reference's
@@ -807,17 +919,17 @@ __host__ __device__ constexpr size_t list_smem(int lcap) {
   return (size_t)LIST_TILE * sizeof(float4) + (size_t)LIST_ATOMS * lcap * (sizeof(int) + sizeof(float));
 }
 
-template <bool IMG>
-__device__ __forceinline__ void list_cells_item(const Arena& A, const BlockMap& C, int b, int part, float4* cf,
-                                                int* stage, float* stage_rd, int* nb_start, int* nb_pref,
-                                                double3* nb_sh, int* boff) {
+// (TILE: candidates staged at a time; the CTA takes the atom passes part,
+// part + nparts, ... of the cells [c0, c1) of system s)
+template <bool IMG, int TILE>
+__device__ __forceinline__ void list_cells_item(const Arena& A, int s, const SysDev& S, int c0, int c1, int part,
+                                                int nparts, float4* cf, int* stage, float* stage_rd, int* nb_start,
+                                                int* nb_pref, double3* nb_sh, int* boff) {
   const int warp = threadIdx.x >> 5, ln = threadIdx.x & 31;
   const unsigned FULL = 0xffffffffu;
-  const int s = C.sys[b];
-  const SysDev& S = A.sys[s];
   const ListFrame f = list_frame(S);
   const bool half = S.half != 0;
-  for (int c = C.first[b]; c < C.end[b]; c++) {
+  for (int c = c0; c < c1; c++) {
     const int cnt0 = A.cell_n[c];
     const int a_first = part * LIST_ATOMS;
     if (a_first >= cnt0) continue;  // uniform per CTA
@@ -864,12 +976,12 @@ __device__ __forceinline__ void list_cells_item(const Arena& A, const BlockMap& 
         if (g < own) A.pos_old[j] = p;  // the home cell's atoms: the list's reference positions
       }
     };
-    const bool one = T <= LIST_TILE;  // one tile stays staged for all this CTA's passes
+    const bool one = T <= TILE;  // one tile stays staged for all this CTA's passes
     if (one) {
       stage_tile(0, T);
       __syncthreads();
     }
-    for (int a0 = a_first; a0 < cnt0; a0 += LIST_ATOMS * LIST_SPLIT) {
+    for (int a0 = a_first; a0 < cnt0; a0 += LIST_ATOMS * nparts) {
       const int a = a0 + warp;  // this warp's atom: chain position a of the cell
       const bool act = a < cnt0;
       int i = -1;
@@ -886,8 +998,8 @@ __device__ __forceinline__ void list_cells_item(const Arena& A, const BlockMap& 
       int* row = stage + warp * A.lcap;
       float* rrow = stage_rd + warp * A.lcap;
       int m = 0;
-      for (int t0 = 0; t0 < T; t0 += LIST_TILE) {
-        const int tn = min(LIST_TILE, T - t0);
+      for (int t0 = 0; t0 < T; t0 += TILE) {
+        const int tn = min(TILE, T - t0);
         if (!one) {
           __syncthreads();
           stage_tile(t0, tn);
@@ -925,10 +1037,14 @@ __global__ void __launch_bounds__(BLOCK) k_list_cells(Arena A, BlockMap C) {
   };
   rebuild_items(C.nblk * LIST_SPLIT, live, [&](int w) {
     const int b = w % C.nblk, part = w / C.nblk;
-    if (A.sys[C.sys[b]].list_img)
-      list_cells_item<true>(A, C, b, part, cf, stage, stage_rd, nb_start, nb_pref, nb_sh, boff_sh[warp]);
+    const int s = C.sys[b], c0 = C.first[b], c1 = C.end[b];
+    const SysDev& S = A.sys[s];
+    if (S.list_img)
+      list_cells_item<true, LIST_TILE>(A, s, S, c0, c1, part, LIST_SPLIT, cf, stage, stage_rd, nb_start, nb_pref,
+                                       nb_sh, boff_sh[warp]);
     else
-      list_cells_item<false>(A, C, b, part, cf, stage, stage_rd, nb_start, nb_pref, nb_sh, boff_sh[warp]);
+      list_cells_item<false, LIST_TILE>(A, s, S, c0, c1, part, LIST_SPLIT, cf, stage, stage_rd, nb_start, nb_pref,
+                                        nb_sh, boff_sh[warp]);
   });
 }
 
@@ -953,15 +1069,11 @@ __host__ __device__ constexpr size_t listw_smem(int lcap) {
 }
 
 template <bool IMG, int TILE>
-__device__ __forceinline__ void list_cells_w_item(const Arena& A, const BlockMap& C, int b, float4* cf, int* boff,
+__device__ __forceinline__ void list_cells_w_item(const Arena& A, int s, const SysDev& S, int c, float4* cf, int* boff,
                                                   int* row, float* rrow) {
   constexpr int U = 2;  // loads in flight per lane while staging
-  const int warp = threadIdx.x >> 5, ln = threadIdx.x & 31;
+  const int ln = threadIdx.x & 31;
   const unsigned FULL = 0xffffffffu;
-  const int c = C.first[b] + warp;
-  if (c >= C.end[b]) return;  // warp-uniform
-  const int s = C.sys[b];
-  const SysDev& S = A.sys[s];
   const ListFrame f = list_frame(S);
   const bool half = S.half != 0;
   const int cl = c - S.cell_off;
@@ -1069,7 +1181,10 @@ __global__ void __launch_bounds__(BLOCK, 2) k_list_cells_w(Arena A, BlockMap C) 
       if (!rebuild_block(A, C, b, true)) return false;
       const SysDev& S = A.sys[C.sys[b]];
       return S.list_warp == KIND && (S.list_img != 0) == IMG;
-    }, [&](int b) { list_cells_w_item<IMG, TILE>(A, C, b, cf, boff, row, rrow); });
+    }, [&](int b) {
+      const int c = C.first[b] + warp;
+      if (c < C.end[b]) list_cells_w_item<IMG, TILE>(A, C.sys[b], A.sys[C.sys[b]], c, cf, boff, row, rrow);  // warp-uniform
+    });
 }
 
 // verlet_self / verlet_selfhalf (src/Neighbour.F90:676-811): O(N^2) over the
@@ -1130,7 +1245,7 @@ __global__ void k_count_rebuild(Arena A, const int* sys, int nsys, int in_graph)
 // Six per-system sums (xx yy zz xy xz yz of a tensor): each block sums its
 // threads' values; the system's last block adds the block partials in
 // block order, so the result is the same bits on every run.
-__device__ __forceinline__ void sys6_close(Arena& A, const BlockMap& M, int s, const double w[6], double* dst) {
+__device__ __forceinline__ void sys6_close(const Arena& A, const BlockMap& M, int s, const double w[6], double* dst) {
   double b[6];
 #pragma unroll
   for (int k = 0; k < 6; k++) b[k] = block_sum(w[k]);
@@ -1154,7 +1269,7 @@ __device__ __forceinline__ void sys6_close(Arena& A, const BlockMap& M, int s, c
 // the sum over the full list of vd (x) f vd / r (vd = r_j - r_i), the
 // virial inq_virial (Inq_Properties.F90:439-527) builds from local and
 // ghost atoms.
-__device__ __forceinline__ void virial_close(Arena& A, const BlockMap& M, int s, const double w[6]) {
+__device__ __forceinline__ void virial_close(const Arena& A, const BlockMap& M, int s, const double w[6]) {
   sys6_close(A, M, s, w, A.st[s].vir);
 }
 
@@ -1279,23 +1394,39 @@ __global__ void k_kin_tensor(Arena A, BlockMap M) {
 // ------------------------------------------------------------------ SMA-TB
 // Per species-pair constants of the FP64 kernels.
 struct SmFP64 {
-  double A, eps2, p, q, r0, rci, rce, b1, b2, b3, r1, r2, r3, pr0, q2r0;
+  double A, eps2, rci, rce, b1, b2, b3, r1, r2, r3;
+  double p, kp, q2, kq;  // exp(-p (r/r0 - 1)) = exp(kp r + p), exp(-2q (r/r0 - 1)) = exp(kq r + q2)
+  // the force pass's constants with the unit ev_ui folded in: 2 A p/r0,
+  // xi^2/2 2q/r0; the tail derivatives' coefficients 5 b1, 4 b2, 3 b3 and
+  // 2 (5 r1, 4 r2, 3 r3)
+  double c1e, c2e, dp5, dp4, dp3, dr5, dr4, dr3;
+  int wide, pad;  // the exponents leave exp_mid's range for some r <= rce
 };
 __device__ __forceinline__ SmFP64 sm_load(const PairP& P) {
   SmFP64 c;
-  c.A = P.v[0];
+  const double A = P.v[0], p = P.v[2], q = P.v[3], r0 = P.v[4], e = EV_UI;
+  c.A = A;
   c.eps2 = P.v[1] * P.v[1];
-  c.p = P.v[2];
-  c.q = P.v[3];
-  c.r0 = P.v[4];
   c.rci = P.v[5];
   c.rce = P.v[6];
   c.b1 = P.v[7]; c.b2 = P.v[8]; c.b3 = P.v[9];
   c.r1 = P.v[10]; c.r2 = P.v[11]; c.r3 = P.v[12];
-  c.pr0 = P.v[2] / P.v[4];
-  c.q2r0 = 2.0 * P.v[3] / P.v[4];
+  c.p = p;
+  c.kp = -p / r0;
+  c.q2 = 2.0 * q;
+  c.kq = -2.0 * q / r0;
+  c.c1e = 2.0 * A * p / r0 * e;
+  c.c2e = c.eps2 * q / r0 * e;
+  c.dp5 = 5.0 * c.b1 * e; c.dp4 = 4.0 * c.b2 * e; c.dp3 = 3.0 * c.b3 * e;
+  c.dr5 = 10.0 * c.r1 * e; c.dr4 = 8.0 * c.r2 * e; c.dr3 = 6.0 * c.r3 * e;
+  const double ext = fmax(fmax(fabs(p), fabs(c.q2)), fmax(fabs(fma(c.kp, c.rce, p)), fabs(fma(c.kq, c.rce, c.q2))));
+  c.wide = !(ext < EXP_MID);
+  c.pad = 0;
   return c;
 }
+
+// the exponentials of a pair: exp_mid inside its range, else the library's
+__device__ __forceinline__ double sm_exp(const SmFP64& c, double x) { return c.wide ? exp(x) : exp_mid(x); }
 
 template <int K>
 __device__ __forceinline__ double lane_sum(double v) {
@@ -1316,38 +1447,85 @@ __device__ __forceinline__ float lane_sumf(float v) {
 // gather latency, not arithmetic).
 constexpr int UNR = 4;
 
-// list slots m0, m0+K, ... (UNR of them) of atom i; slots past nn, and ids
-// outside the arena (never gather outside it), read as -1
-template <int K, int N>
-__device__ __forceinline__ void list_group(const Arena& A, int i, int nn, int m0, int (&jj)[N]) {
+// Where a force body finds an atom's list and its neighbours' records: here
+// the arena.  (team.cuh has the shared-memory counterpart.)
+template <bool NC>
+struct SrcArena {
+  const Arena& A;
+  int lk;           // live_band
+  const int4* fxp;  // the records that are gathered, fixed-point and FP64
+  const double4* pos;
+  __device__ __forceinline__ int count(int i) const { return live_entries<NC>(A, lk, i, min(A.nn[i], A.lcap)); }
+  // list slot m of atom i; ids outside the arena (never gather outside it) read as -1
+  __device__ __forceinline__ int id(int i, int m) const {
+    const int* p = &A.flist[(size_t)m * A.cap + i];
+    const int j = NC ? __ldg(p) : *p;
+    return (unsigned)j < (unsigned)A.cap ? j : -1;
+  }
+  __device__ __forceinline__ int type(int j) const { return A.type[j]; }
+  // fixed-point and FP64 records: position and species; position and 1/sqrt(rho)
+  __device__ __forceinline__ int4 fx(int j) const { return fxp[j]; }
+  __device__ __forceinline__ int4 fxe(int j) const { return A.fxe[j]; }
+  __device__ __forceinline__ double4 x(int j) const { return pos[j]; }
+  __device__ __forceinline__ double4 xe(int j) const { return A.pose[j]; }
+  __device__ __forceinline__ double band(int i) const { return A.band[i]; }
+  __device__ __forceinline__ double eb(int i) const { return A.eband[i]; }
+  __device__ __forceinline__ float ebf(int i) const { return A.ebandf[i]; }
+  // the density pass's results, with the records the force pass gathers
+  __device__ __forceinline__ void put_rho64(int i, double band) const {
+    A.band[i] = band;
+    const double eb = 1.0 / sqrt(band);
+    A.eband[i] = eb;
+    A.ebandf[i] = (float)eb;
+    const double4 xi = pos[i];
+    A.pose[i] = make_double4(xi.x, xi.y, xi.z, eb);  // one gather per neighbour in the force pass
+  }
+  __device__ __forceinline__ void put_rho32(int i, double band) const {
+    A.band[i] = band;
+    const double eb = 1.0 / sqrt(band);
+    A.eband[i] = eb;
+    const float ebf = (float)eb;
+    A.ebandf[i] = ebf;
+    const int4 xi = fxp[i];
+    A.fxe[i] = make_int4(xi.x, xi.y, xi.z, __float_as_int(ebf));  // one gather per neighbour
+  }
+};
+__device__ __forceinline__ SrcArena<true> src_arena(const Arena& A, const SysDev& S, const SysState& st) {
+  return SrcArena<true>{A, live_band(S, st), A.fxp, A.pos};
+}
+
+// list slots m0, m0+K, ... (N of them) of atom i; slots past nn read as -1
+template <int K, int N, class Src>
+__device__ __forceinline__ void list_group(const Src& src, int i, int nn, int m0, int (&jj)[N]) {
 #pragma unroll
   for (int u = 0; u < N; u++) {
-    int m = m0 + u * K;
-    int j = m < nn ? __ldg(&A.flist[(size_t)m * A.cap + i]) : -1;
-    jj[u] = (unsigned)j < (unsigned)A.cap ? j : -1;
+    const int m = m0 + u * K;
+    jj[u] = m < nn ? src.id(i, m) : -1;
   }
 }
 
 // The indices of the next group are loaded while the current group is
 // gathered and computed, so a lane waits on one memory latency per group
-// instead of two (list load, then the gathers it feeds).
-#define PAIR_LOOP_BEGIN(GATHER_T, GATHER)                                      \
-  int jn_[UNR];                                                               \
-  list_group<K>(A, i, nn, lane, jn_);                                         \
-  for (int m0 = lane; m0 < nn; m0 += UNR * K) {                               \
-    int jj[UNR];                                                              \
-    _Pragma("unroll") for (int u = 0; u < UNR; u++) jj[u] = jn_[u];           \
-    GATHER_T gj[UNR];                                                         \
-    _Pragma("unroll") for (int u = 0; u < UNR; u++) if (jj[u] >= 0) gj[u] = GATHER(jj[u]); \
-    list_group<K>(A, i, nn, m0 + UNR * K, jn_);                               \
-    _Pragma("unroll") for (int u = 0; u < UNR; u++) {                         \
-      if (jj[u] < 0) continue;                                                \
-      const int j = jj[u];                                                    \
-      (void)j;
-#define PAIR_LOOP_END \
-    }                 \
+// instead of two (list load, then the gathers it feeds).  An empty slot
+// (jj < 0) gathers the atom itself and is masked.
+template <int K, int N, class Body, class Src, class Gather, class T>
+__device__ __forceinline__ void pair_groups(const Src& src, int i, int nn, int lane, const T& self, Gather gather,
+                                            Body body) {
+  int jn[N];
+  list_group<K>(src, i, nn, lane, jn);
+  for (int m0 = lane; m0 < nn; m0 += N * K) {
+    int jj[N];
+    T gj[N];
+#pragma unroll
+    for (int u = 0; u < N; u++) {
+      jj[u] = jn[u];
+      gj[u] = self;
+      if (jj[u] >= 0) gj[u] = gather(jj[u]);
+    }
+    list_group<K>(src, i, nn, m0 + N * K, jn);
+    body(jj, gj);
   }
-
+}
 
 // smatb_preinteraction (src/TB.F90:367-455), FP64: rho_i = sum_j
 //   xi^2 exp(-2q(r/r0-1))            r <  rci
@@ -1359,6 +1537,40 @@ __device__ __forceinline__ const SmFP64* sm_table(const Arena& A, const SysDev& 
   return sh;
 }
 
+constexpr int UNR_R64 = 4, UNR_F64 = 2;  // pairs of a group in the two FP64 passes
+template <int K, class Src>
+__device__ __forceinline__ void rho_fp64_body(const Src& src, const SysDev& S, const SmFP64* tab, int i, int lane,
+                                              bool act) {
+  double band = 0.0;
+  if (act) {
+    const double4 xi = src.x(i);
+    const bool one = S.ntypes == 1;
+    const SmFP64* row = tab + (one ? 0 : src.type(i) * S.ntypes);
+    const int nn = src.count(i);
+    const ImgTest img = img_test(S);
+    auto body = [&](const int (&jj)[UNR_R64], const double4 (&gj)[UNR_R64]) {
+      double v[UNR_R64][3];
+      vd_fp64(S, img, xi, gj, v);
+      // branch-free: both regimes are evaluated and selected, so the group's
+      // chains interleave
+#pragma unroll
+      for (int u = 0; u < UNR_R64; u++) {
+        const SmFP64& c = row[one || jj[u] < 0 ? 0 : src.type(jj[u])];
+        double rinv;
+        const double dr = sqrt_pos(v[u][0] * v[u][0] + v[u][1] * v[u][1] + v[u][2] * v[u][2], rinv);
+        const double bin = c.eps2 * sm_exp(c, fma(c.kq, dr, c.q2));
+        const double d = dr - c.rce;
+        const double bt = fma(fma(c.b1, d, c.b2), d, c.b3) * (d * d * d);
+        const double banda = dr < c.rci ? bin : bt * bt;
+        band += jj[u] < 0 || dr > c.rce ? 0.0 : banda;
+      }
+    };
+    pair_groups<K, UNR_R64>(src, i, nn, lane, xi, [&](int j) { return src.x(j); }, body);
+  }
+  band = lane_sum<K>(band);
+  if (act && lane == 0) src.put_rho64(i, band);
+}
+
 template <int K>
 __global__ void __launch_bounds__(BLOCK) k_smatb_rho_fp64(Arena A, BlockMap M) {
   int s = blk_sys(M);
@@ -1366,43 +1578,12 @@ __global__ void __launch_bounds__(BLOCK) k_smatb_rho_fp64(Arena A, BlockMap M) {
   const SysDev& S = A.sys[s];
   __shared__ SmFP64 tab_sh[MAXT * MAXT];
   const SmFP64* tab = sm_table(A, S, tab_sh);
-  int i = M.first[blockIdx.x] + threadIdx.x / K;
-  int lane = threadIdx.x % K;
-  bool act = i < M.end[blockIdx.x];
-  double band = 0.0;
-  if (act) {
-    const double4 xi = A.pos[i];
-    const int ti = A.type[i];
-    const int nn = live_entries(A, S, A.st[s], i, min(A.nn[i], A.lcap));
-    const bool one = S.ntypes == 1;
-    auto gat = [&](int j) { return A.pos[j]; };
-    PAIR_LOOP_BEGIN(double4, gat)
-      const SmFP64& c = tab[one ? 0 : ti * S.ntypes + A.type[j]];
-      double v0, v1, v2;
-      vd_fp64(S, xi, gj[u], v0, v1, v2);
-      double dr = sqrt(v0 * v0 + v1 * v1 + v2 * v2);
-      if (dr > c.rce) continue;
-      double banda;
-      if (dr < c.rci) {
-        banda = c.eps2 * exp(-2.0 * c.q * (dr / c.r0 - 1.0));
-      } else {
-        double d = dr - c.rce, d2 = d * d, d3 = d2 * d;
-        banda = (c.b1 * d2 + c.b2 * d + c.b3) * d3;
-        banda = banda * banda;
-      }
-      band += banda;
-    PAIR_LOOP_END
-  }
-  band = lane_sum<K>(band);
-  if (act && lane == 0) {
-    A.band[i] = band;
-    double eb = 1.0 / sqrt(band);
-    A.eband[i] = eb;
-    A.ebandf[i] = (float)eb;
-    const double4 xi = A.pos[i];
-    A.pose[i] = make_double4(xi.x, xi.y, xi.z, eb);  // one gather per neighbour in the force pass
-  }
+  const int i = M.first[blockIdx.x] + threadIdx.x / K;
+  rho_fp64_body<K>(src_arena(A, S, A.st[s]), S, tab, i, threadIdx.x % K, i < M.end[blockIdx.x]);
 }
+
+// an atom's energy from its pair sum and density
+__device__ __forceinline__ double sm_energy(double ep, double band) { return (ep - sqrt(band)) * EV_UI; }
 
 // smatb_interact (src/TB.F90:457-586), FP64, full list (newton off):
 //   r <= rci : factor = 2 A e^{-p(r/r0-1)} p/r0
@@ -1415,66 +1596,65 @@ __global__ void __launch_bounds__(BLOCK) k_smatb_rho_fp64(Arena A, BlockMap M) {
 // VIR: also the pair virial of the system (virial_close); SMA-TB forces are
 // central pair forces, F_i = -sum_j factor_ij vd / r, so W is the pair sum
 // (complete: the reference's TB.F90:548-564 omits the i-side term).
-template <int K, bool VIR, bool STORE = true>
-__device__ __forceinline__ void force_fp64_body(Arena& A, const BlockMap& M, int s, const SysDev& S,
-                                                const SmFP64* tab, int i, int lane, bool act, double4& F) {
+template <int K, bool VIR, bool STORE = true, class Src>
+__device__ __forceinline__ void force_fp64_body(const Src& src, const Arena& A, const BlockMap& M, int s,
+                                                const SysDev& S, const SmFP64* tab, int i, int lane, bool act,
+                                                double4& F) {
   double f0 = 0, f1 = 0, f2 = 0, ep = 0;
   double w[6] = {0, 0, 0, 0, 0, 0};
   if (act) {
-    const double4 xi = A.pos[i];
-    const int ti = A.type[i];
-    const double ebi = A.eband[i];
-    const int nn = live_entries(A, S, A.st[s], i, min(A.nn[i], A.lcap));
+    const double4 xi = src.x(i);
+    const double ebi = src.eb(i);
     const bool one = S.ntypes == 1;
-    auto gat = [&](int j) { return A.pose[j]; };
-    PAIR_LOOP_BEGIN(double4, gat)
-      const SmFP64& c = tab[one ? 0 : ti * S.ntypes + A.type[j]];
-      double v0, v1, v2;
-      vd_fp64(S, xi, gj[u], v0, v1, v2);
-      double dr = sqrt(v0 * v0 + v1 * v1 + v2 * v2);
-      if (dr > c.rce) continue;
-      double factor, repul;
-      double ebs = ebi + gj[u].w;
-      if (dr <= c.rci) {
-        double x = dr / c.r0 - 1.0;
-        repul = c.A * exp(-c.p * x);
-        factor = 2.0 * repul * c.pr0 - c.eps2 * 0.5 * exp(-2.0 * c.q * x) * c.q2r0 * ebs;
-      } else {
-        double d = dr - c.rce, d2 = d * d, d3 = d2 * d, d4 = d3 * d;
-        double P = (c.b1 * d2 + c.b2 * d + c.b3) * d3;
-        double dP = 5.0 * c.b1 * d4 + 4.0 * c.b2 * d3 + 3.0 * c.b3 * d2;
-        double dR = 5.0 * c.r1 * d4 + 4.0 * c.r2 * d3 + 3.0 * c.r3 * d2;
-        factor = P * dP * ebs - 2.0 * dR;
-        repul = (c.r1 * d2 + c.r2 * d + c.r3) * d3;
+    const SmFP64* row = tab + (one ? 0 : src.type(i) * S.ntypes);
+    const int nn = src.count(i);
+    const ImgTest img = img_test(S);
+    auto body = [&](const int (&jj)[UNR_F64], const double4 (&gj)[UNR_F64]) {
+      double v[UNR_F64][3];
+      vd_fp64(S, img, xi, gj, v);
+#pragma unroll
+      for (int u = 0; u < UNR_F64; u++) {
+        const SmFP64& c = row[one || jj[u] < 0 ? 0 : src.type(jj[u])];
+        double rinv;
+        const double dr = sqrt_pos(v[u][0] * v[u][0] + v[u][1] * v[u][1] + v[u][2] * v[u][2], rinv);
+        const bool off = jj[u] < 0 || dr > c.rce;
+        const double ebs = ebi + gj[u].w;
+        const double e1 = sm_exp(c, fma(c.kp, dr, c.p)), e2 = sm_exp(c, fma(c.kq, dr, c.q2));
+        const double d = dr - c.rce, d2 = d * d, d3 = d2 * d;
+        const double P = fma(fma(c.b1, d, c.b2), d, c.b3) * d3;
+        const double dPe = fma(fma(c.dp5, d, c.dp4), d, c.dp3) * d2;
+        const double dRe = fma(fma(c.dr5, d, c.dr4), d, c.dr3) * d2;
+        const bool inner = dr <= c.rci;
+        // factor carries ev_ui
+        const double factor = inner ? c.c1e * e1 - c.c2e * e2 * ebs : P * dPe * ebs - dRe;
+        const double repul = inner ? c.A * e1 : fma(fma(c.r1, d, c.r2), d, c.r3) * d3;
+        const double fr = off ? 0.0 : factor * rinv;
+        f0 -= fr * v[u][0];
+        f1 -= fr * v[u][1];
+        f2 -= fr * v[u][2];
+        ep += off ? 0.0 : repul;
+        if constexpr (VIR) {
+          const double h = 0.5 * fr;
+          w[0] += h * v[u][0] * v[u][0];
+          w[1] += h * v[u][1] * v[u][1];
+          w[2] += h * v[u][2] * v[u][2];
+          w[3] += h * v[u][0] * v[u][1];
+          w[4] += h * v[u][0] * v[u][2];
+          w[5] += h * v[u][1] * v[u][2];
+        }
       }
-      double fr = factor * EV_UI / dr;
-      f0 -= fr * v0;
-      f1 -= fr * v1;
-      f2 -= fr * v2;
-      ep += repul;
-      if constexpr (VIR) {
-        const double h = 0.5 * fr;
-        w[0] += h * v0 * v0;
-        w[1] += h * v1 * v1;
-        w[2] += h * v2 * v2;
-        w[3] += h * v0 * v1;
-        w[4] += h * v0 * v2;
-        w[5] += h * v1 * v2;
-      }
-    PAIR_LOOP_END
+    };
+    pair_groups<K, UNR_F64>(src, i, nn, lane, xi, [&](int j) { return src.xe(j); }, body);
   }
   f0 = lane_sum<K>(f0);
   f1 = lane_sum<K>(f1);
   f2 = lane_sum<K>(f2);
   ep = lane_sum<K>(ep);
-  if (act && lane == 0) {
-    const double e = (ep - sqrt(A.band[i])) * EV_UI;
-    if constexpr (STORE) {
-      F = make_double4(f0, f1, f2, 0.0);
-      A.force[i] = F;
-      A.epot[i] = e;
-    } else {
-      F = make_double4(f0, f1, f2, e);
+  F = make_double4(f0, f1, f2, ep);  // in every lane
+  if constexpr (STORE) {
+    if (act && lane == 0) {
+      A.force[i] = make_double4(f0, f1, f2, 0.0);
+      A.epot[i] = sm_energy(ep, src.band(i));
     }
   }
   if constexpr (VIR) virial_close(A, M, s, w);
@@ -1489,7 +1669,7 @@ __global__ void __launch_bounds__(BLOCK) k_smatb_force_fp64(Arena A, BlockMap M)
   const SmFP64* tab = sm_table(A, S, tab_sh);
   const int i = M.first[blockIdx.x] + threadIdx.x / K;
   double4 F;
-  force_fp64_body<K, VIR>(A, M, s, S, tab, i, threadIdx.x % K, i < M.end[blockIdx.x], F);
+  force_fp64_body<K, VIR>(src_arena(A, S, A.st[s]), A, M, s, S, tab, i, threadIdx.x % K, i < M.end[blockIdx.x], F);
 }
 
 // ---- mixed precision: FP32 pair math, FP64 accumulation.
@@ -1498,12 +1678,13 @@ __global__ void __launch_bounds__(BLOCK) k_smatb_force_fp64(Arena A, BlockMap M)
 struct SmF32 {
   float kp, kq, r0;    // e1 = 2^(kp (r0 - r)) = exp(-p(r/r0-1)),
                        // e2 = 2^(kq (r0 - r)) = exp(-2q(r/r0-1)); r0 - r is exact
-  float A, eps2, c1, c2;
+  float A, eps2;
   float rci, rce, rci2, rce2;
   float b1, b2, b3, r1, r2, r3;
   // the force pass's constants with the unit ev_ui folded in: c1, c2; the
   // tail derivatives' coefficients 5 b1, 4 b2, 3 b3 and 2 (5 r1, 4 r2, 3 r3)
-  float c1e, c2e, dp5, dp4, dp3, dr5, dr4, dr3;
+  // (nc2e and ndr*: negated, for fused multiply-adds without a sign change)
+  float c1e, nc2e, dp5, dp4, dp3, ndr5, ndr4, ndr3;
 };
 __device__ __forceinline__ SmF32 smf_load(const PairP& P) {
   const double log2e = 1.4426950408889634;
@@ -1514,8 +1695,6 @@ __device__ __forceinline__ SmF32 smf_load(const PairP& P) {
   c.r0 = (float)r0;
   c.A = (float)A;
   c.eps2 = (float)(xi * xi);
-  c.c1 = (float)(2.0 * A * p / r0);          // 2 A p/r0 (times e1)
-  c.c2 = (float)(xi * xi * q / r0);          // xi^2/2 * 2q/r0 (times e2 * ebs)
   c.rci = (float)P.v[5];
   c.rce = (float)P.v[6];
   c.rci2 = (float)(P.v[5] * P.v[5]);
@@ -1524,9 +1703,9 @@ __device__ __forceinline__ SmF32 smf_load(const PairP& P) {
   c.r1 = (float)P.v[10]; c.r2 = (float)P.v[11]; c.r3 = (float)P.v[12];
   const double e = EV_UI;
   c.c1e = (float)(2.0 * A * p / r0 * e);
-  c.c2e = (float)(xi * xi * q / r0 * e);
+  c.nc2e = (float)(-xi * xi * q / r0 * e);
   c.dp5 = (float)(5.0 * P.v[7] * e); c.dp4 = (float)(4.0 * P.v[8] * e); c.dp3 = (float)(3.0 * P.v[9] * e);
-  c.dr5 = (float)(10.0 * P.v[10] * e); c.dr4 = (float)(8.0 * P.v[11] * e); c.dr3 = (float)(6.0 * P.v[12] * e);
+  c.ndr5 = (float)(-10.0 * P.v[10] * e); c.ndr4 = (float)(-8.0 * P.v[11] * e); c.ndr3 = (float)(-6.0 * P.v[12] * e);
   return c;
 }
 
@@ -1548,10 +1727,44 @@ __device__ __forceinline__ float ex2f(float x) {
 
 // r = sqrt(r2) and 1/r from one MUFU rsqrt plus a Newton step on r
 // (accurate to ~1 ulp without the IEEE sqrt / rcp instruction sequences)
+__device__ __forceinline__ float rsqrt_mufu(float x) {
+  float y;
+  asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
+}
 __device__ __forceinline__ float sqrt_nr(float r2, float& rinv) {
-  rinv = rsqrtf(r2);
+  rinv = rsqrt_mufu(r2);
   float r = r2 * rinv;
   return fmaf(0.5f * rinv, fmaf(-r, r, r2), r);
+}
+
+// ---- two pairs at a time: the packed FP32 instructions do two operations per
+// issue slot, and the pair loops are bound by issue slots (a density pass
+// over 256k atoms issued 78 instructions per list slot, 81 % of the slots of
+// its time), not by the FMA pipe (36 % busy).  Each half rounds as the
+// scalar operation does.
+__device__ __forceinline__ float2 f2(float a, float b) { return make_float2(a, b); }
+__device__ __forceinline__ float2 f2(float a) { return make_float2(a, a); }
+__device__ __forceinline__ float2 operator*(float2 a, float2 b) { return __fmul2_rn(a, b); }
+__device__ __forceinline__ float2 operator+(float2 a, float2 b) { return __fadd2_rn(a, b); }
+__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) { return __ffma2_rn(a, b, c); }
+
+// the pair vectors of two neighbours
+__device__ __forceinline__ void vd_fx2(const SysDev& S, int4 a, int4 b0, int4 b1, float2 (&v)[3]) {
+  const float2 x = f2((float)(b0.x - a.x), (float)(b1.x - a.x)), y = f2((float)(b0.y - a.y), (float)(b1.y - a.y)),
+               z = f2((float)(b0.z - a.z), (float)(b1.z - a.z));
+  v[0] = fma2(x, f2(S.fx_inv[0]), x * f2(S.fx_inv_lo[0]));
+  v[1] = fma2(y, f2(S.fx_inv[1]), y * f2(S.fx_inv_lo[1]));
+  v[2] = fma2(z, f2(S.fx_inv[2]), z * f2(S.fx_inv_lo[2]));
+}
+__device__ __forceinline__ float2 norm2(const float2 (&v)[3]) {
+  return fma2(v[2], v[2], fma2(v[1], v[1], v[0] * v[0]));
+}
+// sqrt_nr of both halves
+__device__ __forceinline__ float2 sqrt_nr2(float2 r2, float2& rinv) {
+  rinv = f2(rsqrt_mufu(r2.x), rsqrt_mufu(r2.y));
+  const float2 r = r2 * rinv;
+  return fma2(rinv * f2(-0.5f), fma2(r, r, r2 * f2(-1.0f)), r);
 }
 
 // Mixed kernels sum the FP32 pair terms of one group (UNR_R pairs in the
@@ -1573,6 +1786,44 @@ __device__ __forceinline__ const SmF32* smf_table(const Arena& A, const SysDev& 
 
 // MINB > 1 asks the compiler to fit MINB blocks per SM (fewer registers,
 // more warps to hide gather latency); the autotuner tries both.
+template <int K, bool ONE, class Src>
+__device__ __forceinline__ void rho_mixed_body(const Src& src, const Arena& A, const SysDev& S, const SmF32* tab, int i,
+                                               int lane, bool act) {
+  double band = 0.0;
+  if (act) {
+    const int4 xi = src.fx(i);
+    const int nn = src.count(i);
+    const SmF32 c1 = ONE ? smf_load(A.prm[S.param_off]) : SmF32{};
+    auto body = [&](const int (&jj)[UNR_R], const int4 (&gj)[UNR_R]) {
+      float grp = 0.0f;
+      // branch-free: both regimes are evaluated and selected, so the
+      // group's pairs interleave (a warp's lanes would run both anyway)
+#pragma unroll
+      for (int u = 0; u < UNR_R; u += 2) {
+        const SmF32& a = ONE ? c1 : tab[xi.w * S.ntypes + gj[u].w];
+        const SmF32& b = ONE ? c1 : tab[xi.w * S.ntypes + gj[u + 1].w];
+        float2 v[3], rinv;
+        vd_fx2(S, xi, gj[u], gj[u + 1], v);
+        float2 r2 = norm2(v);
+        const bool oka = jj[u] >= 0 && !(r2.x > a.rce2), okb = jj[u + 1] >= 0 && !(r2.y > b.rce2);
+        r2 = f2(oka ? r2.x : a.rce2, okb ? r2.y : b.rce2);
+        const float2 dr = sqrt_nr2(r2, rinv);
+        const float2 ex = f2(a.kq, b.kq) * fma2(dr, f2(-1.0f), f2(a.r0, b.r0));
+        const float2 bin = f2(a.eps2, b.eps2) * f2(ex2f(ex.x), ex2f(ex.y));
+        const float2 d = dr + f2(-a.rce, -b.rce);
+        float2 bt = fma2(fma2(f2(a.b1, b.b1), d, f2(a.b2, b.b2)), d, f2(a.b3, b.b3)) * (d * d * d);
+        bt = bt * bt;
+        grp += oka ? (dr.x < a.rci ? bin.x : bt.x) : 0.0f;
+        grp += okb ? (dr.y < b.rci ? bin.y : bt.y) : 0.0f;
+      }
+      band += (double)grp;
+    };
+    pair_groups<K, UNR_R>(src, i, nn, lane, xi, [&](int j) { return src.fx(j); }, body);
+  }
+  band = lane_sum<K>(band);
+  if (act && lane == 0) src.put_rho32(i, band);
+}
+
 template <int K, bool ONE, int MINB>
 __global__ void __launch_bounds__(BLOCK, MINB) k_smatb_rho_mixed(Arena A, BlockMap M) {
   int s = blk_sys(M);
@@ -1580,156 +1831,86 @@ __global__ void __launch_bounds__(BLOCK, MINB) k_smatb_rho_mixed(Arena A, BlockM
   const SysDev& S = A.sys[s];
   __shared__ SmF32 tab_sh[ONE ? 1 : MAXT * MAXT];
   const SmF32* tab = smf_table<ONE>(A, S, tab_sh);
-  int i = M.first[blockIdx.x] + threadIdx.x / K;
-  int lane = threadIdx.x % K;
-  bool act = i < M.end[blockIdx.x];
-  double band = 0.0;
-  if (act) {
-    const int4 xi = A.fxp[i];
-    const int nn = live_entries(A, S, A.st[s], i, min(A.nn[i], A.lcap));
-    const SmF32 c1 = ONE ? smf_load(A.prm[S.param_off]) : SmF32{};
-    int jn[UNR_R];
-    list_group<K>(A, i, nn, lane, jn);
-    for (int m0 = lane; m0 < nn; m0 += UNR_R * K) {
-      int jj[UNR_R];
-#pragma unroll
-      for (int u = 0; u < UNR_R; u++) jj[u] = jn[u];
-      int4 gj[UNR_R];
-#pragma unroll
-      for (int u = 0; u < UNR_R; u++) {
-        gj[u] = xi;  // an empty slot: a zero pair vector, masked below
-        if (jj[u] >= 0) gj[u] = A.fxp[jj[u]];
-      }
-      list_group<K>(A, i, nn, m0 + UNR_R * K, jn);  // next group's ids, in flight meanwhile
-      float grp = 0.0f;
-      // branch-free: both regimes are evaluated and selected, so the
-      // group's pairs interleave (a warp's lanes would run both anyway)
-#pragma unroll
-      for (int u = 0; u < UNR_R; u++) {
-        const int4 xj = gj[u];
-        const SmF32& c = ONE ? c1 : tab[xi.w * S.ntypes + xj.w];
-        float v0, v1, v2;
-        vd_fx(S, xi, xj, v0, v1, v2);
-        const float r2 = v0 * v0 + v1 * v1 + v2 * v2;
-        const bool ok = jj[u] >= 0 && !(r2 > c.rce2);
-        float rinv;
-        const float dr = sqrt_nr(ok ? r2 : c.rce2, rinv);
-        const float bin = c.eps2 * ex2f(c.kq * (c.r0 - dr));
-        const float d = dr - c.rce, d3 = d * d * d;
-        float bt = fmaf(fmaf(c.b1, d, c.b2), d, c.b3) * d3;
-        bt = bt * bt;
-        const float banda = dr < c.rci ? bin : bt;
-        grp += ok ? banda : 0.0f;
-      }
-      band += (double)grp;
-    }
-  }
-  band = lane_sum<K>(band);
-  if (act && lane == 0) {
-    A.band[i] = band;
-    double eb = 1.0 / sqrt(band);
-    A.eband[i] = eb;
-    const float ebf = (float)eb;
-    A.ebandf[i] = ebf;
-    const int4 xi = A.fxp[i];
-    A.fxe[i] = make_int4(xi.x, xi.y, xi.z, __float_as_int(ebf));  // one gather per neighbour
-  }
+  const int i = M.first[blockIdx.x] + threadIdx.x / K;
+  rho_mixed_body<K, ONE>(src_arena(A, S, A.st[s]), A, S, tab, i, threadIdx.x % K, i < M.end[blockIdx.x]);
 }
 
 // The force pass for one thread's lane of atom i (K lanes per atom); lane 0
 // stores the force and energy and returns the force in F (STORE=false:
-// stores nothing and returns the energy in F.w, for the caller to store).
+// stores nothing); F.w is the pair sum of the energy.
 // VIR: also the pair virial, FP32 per pair and group, FP64 per atom and system.
-template <int K, bool ONE, bool VIR, bool STORE = true>
-__device__ __forceinline__ void force_mixed_body(Arena& A, const BlockMap& M, int s, const SysDev& S,
-                                                 const SmF32* tab, int i, int lane, bool act, double4& F) {
-  double f0 = 0, f1 = 0, f2 = 0, ep = 0;
+template <int K, bool ONE, bool VIR, bool STORE = true, class Src>
+__device__ __forceinline__ void force_mixed_body(const Src& src, const Arena& A, const BlockMap& M, int s,
+                                                 const SysDev& S, const SmF32* tab, int i, int lane, bool act,
+                                                 double4& F) {
+  double f0 = 0, f1 = 0, f2_ = 0, ep = 0;
   double w[6] = {0, 0, 0, 0, 0, 0};
   if (act) {
-    const int4 xi = A.fxp[i];
-    const float ebi = A.ebandf[i];
-    const int nn = live_entries(A, S, A.st[s], i, min(A.nn[i], A.lcap));
+    const int4 xi = src.fx(i);
+    const float2 ebi = f2(src.ebf(i));
+    const int nn = src.count(i);
     const SmF32 c1 = ONE ? smf_load(A.prm[S.param_off]) : SmF32{};
     const int ti = xi.w;
-    int jn[UNR_F];
-    list_group<K>(A, i, nn, lane, jn);
-    for (int m0 = lane; m0 < nn; m0 += UNR_F * K) {
-      int jj[UNR_F];
-#pragma unroll
-      for (int u = 0; u < UNR_F; u++) jj[u] = jn[u];
-      int4 gj[UNR_F];
-      int tj[UNR_F];
-#pragma unroll
-      for (int u = 0; u < UNR_F; u++) {
-        gj[u] = make_int4(xi.x, xi.y, xi.z, 0);  // an empty slot: a zero pair vector, masked below
-        tj[u] = 0;
-        if (jj[u] >= 0) {
-          gj[u] = A.fxe[jj[u]];
-          if (!ONE) tj[u] = A.type[jj[u]];
-        }
-      }
-      list_group<K>(A, i, nn, m0 + UNR_F * K, jn);  // next group's ids, in flight meanwhile
+    auto body = [&](const int (&jj)[UNR_F], const int4 (&gj)[UNR_F]) {
       float g0 = 0.0f, g1 = 0.0f, g2 = 0.0f, ge = 0.0f;
       float gw[6] = {0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f};
       // branch-free: both regimes are evaluated and selected, so the
       // group's pairs interleave (a warp's lanes would run both anyway)
 #pragma unroll
-      for (int u = 0; u < UNR_F; u++) {
-        const int4 xj = gj[u];
-        const SmF32& c = ONE ? c1 : tab[ti * S.ntypes + tj[u]];
-        float v0, v1, v2;
-        vd_fx(S, xi, xj, v0, v1, v2);
-        const float r2 = v0 * v0 + v1 * v1 + v2 * v2;
-        const bool ok = jj[u] >= 0 && !(r2 > c.rce2);
-        float rinv;
-        const float dr = sqrt_nr(ok ? r2 : c.rce2, rinv);
-        const float ebs = ebi + __int_as_float(xj.w);
-        const float x = c.r0 - dr;
-        const float e1 = ex2f(c.kp * x);
-        const float e2 = ex2f(c.kq * x);
+      for (int u = 0; u < UNR_F; u += 2) {
+        const SmF32& a = ONE ? c1 : tab[ti * S.ntypes + (jj[u] < 0 ? 0 : src.type(jj[u]))];
+        const SmF32& b = ONE ? c1 : tab[ti * S.ntypes + (jj[u + 1] < 0 ? 0 : src.type(jj[u + 1]))];
+        float2 v[3], rinv;
+        vd_fx2(S, xi, gj[u], gj[u + 1], v);
+        float2 r2 = norm2(v);
+        const bool oka = jj[u] >= 0 && !(r2.x > a.rce2), okb = jj[u + 1] >= 0 && !(r2.y > b.rce2);
+        r2 = f2(oka ? r2.x : a.rce2, okb ? r2.y : b.rce2);
+        const float2 dr = sqrt_nr2(r2, rinv);
+        const float2 ebs = ebi + f2(__int_as_float(gj[u].w), __int_as_float(gj[u + 1].w));
+        const float2 x = fma2(dr, f2(-1.0f), f2(a.r0, b.r0));
+        const float2 xp = f2(a.kp, b.kp) * x, xq = f2(a.kq, b.kq) * x;
+        const float2 e1 = f2(ex2f(xp.x), ex2f(xp.y)), e2 = f2(ex2f(xq.x), ex2f(xq.y));
         // the tail polynomials in Horner form; factor carries ev_ui
-        const float d = dr - c.rce, d2 = d * d, d3 = d2 * d;
-        const float P = fmaf(fmaf(c.b1, d, c.b2), d, c.b3) * d3;
-        const float dPe = fmaf(fmaf(c.dp5, d, c.dp4), d, c.dp3) * d2;  // ev_ui P'
-        const float dRe = fmaf(fmaf(c.dr5, d, c.dr4), d, c.dr3) * d2;  // 2 ev_ui R'
-        const bool inner = dr <= c.rci;
-        const float factor = inner ? c.c1e * e1 - c.c2e * e2 * ebs : P * dPe * ebs - dRe;
-        const float repul = ok ? (inner ? c.A * e1 : fmaf(fmaf(c.r1, d, c.r2), d, c.r3) * d3) : 0.0f;
-        const float fr = ok ? factor * rinv : 0.0f;
-        g0 = fmaf(fr, v0, g0);
-        g1 = fmaf(fr, v1, g1);
-        g2 = fmaf(fr, v2, g2);
-        ge += repul;
+        const float2 d = dr + f2(-a.rce, -b.rce), d2 = d * d, d3 = d2 * d;
+        const float2 P = fma2(fma2(f2(a.b1, b.b1), d, f2(a.b2, b.b2)), d, f2(a.b3, b.b3)) * d3;
+        const float2 dPe = fma2(fma2(f2(a.dp5, b.dp5), d, f2(a.dp4, b.dp4)), d, f2(a.dp3, b.dp3)) * d2;  // ev_ui P'
+        const float2 ndRe = fma2(fma2(f2(a.ndr5, b.ndr5), d, f2(a.ndr4, b.ndr4)), d, f2(a.ndr3, b.ndr3)) * d2;
+        const float2 Rt = fma2(fma2(f2(a.r1, b.r1), d, f2(a.r2, b.r2)), d, f2(a.r3, b.r3)) * d3;
+        const float2 fin = fma2(f2(a.c1e, b.c1e), e1, f2(a.nc2e, b.nc2e) * e2 * ebs);
+        const float2 ftl = fma2(P * dPe, ebs, ndRe), Ri = f2(a.A, b.A) * e1;
+        const bool ina = dr.x <= a.rci, inb = dr.y <= b.rci;
+        float2 fr = f2(ina ? fin.x : ftl.x, inb ? fin.y : ftl.y) * rinv;
+        fr = f2(oka ? fr.x : 0.0f, okb ? fr.y : 0.0f);
+        ge += oka ? (ina ? Ri.x : Rt.x) : 0.0f;
+        ge += okb ? (inb ? Ri.y : Rt.y) : 0.0f;
+        g0 = fmaf(fr.y, v[0].y, fmaf(fr.x, v[0].x, g0));
+        g1 = fmaf(fr.y, v[1].y, fmaf(fr.x, v[1].x, g1));
+        g2 = fmaf(fr.y, v[2].y, fmaf(fr.x, v[2].x, g2));
         if constexpr (VIR) {
-          const float h = 0.5f * fr;
-          gw[0] += h * v0 * v0;
-          gw[1] += h * v1 * v1;
-          gw[2] += h * v2 * v2;
-          gw[3] += h * v0 * v1;
-          gw[4] += h * v0 * v2;
-          gw[5] += h * v1 * v2;
+          const float2 h = fr * f2(0.5f);
+          const float2 hx = h * v[0], hy = h * v[1], hz = h * v[2];
+          const float2 q[6] = {hx * v[0], hy * v[1], hz * v[2], hx * v[1], hx * v[2], hy * v[2]};
+          for (int k = 0; k < 6; k++) gw[k] += q[k].x + q[k].y;
         }
       }
       f0 -= (double)g0;
       f1 -= (double)g1;
-      f2 -= (double)g2;
+      f2_ -= (double)g2;
       ep += (double)ge;
       if constexpr (VIR)
         for (int k = 0; k < 6; k++) w[k] += (double)gw[k];
-    }
+    };
+    pair_groups<K, UNR_F>(src, i, nn, lane, xi, [&](int j) { return src.fxe(j); }, body);
   }
   f0 = lane_sum<K>(f0);
   f1 = lane_sum<K>(f1);
-  f2 = lane_sum<K>(f2);
+  f2_ = lane_sum<K>(f2_);
   ep = lane_sum<K>(ep);
-  if (act && lane == 0) {
-    const double e = (ep - sqrt(A.band[i])) * EV_UI;
-    if constexpr (STORE) {
-      F = make_double4(f0, f1, f2, 0.0);
-      A.force[i] = F;
-      A.epot[i] = e;
-    } else {
-      F = make_double4(f0, f1, f2, e);
+  F = make_double4(f0, f1, f2_, ep);  // in every lane
+  if constexpr (STORE) {
+    if (act && lane == 0) {
+      A.force[i] = make_double4(f0, f1, f2_, 0.0);
+      A.epot[i] = sm_energy(ep, src.band(i));
     }
   }
   if constexpr (VIR) virial_close(A, M, s, w);
@@ -1744,7 +1925,7 @@ __global__ void __launch_bounds__(BLOCK, MINB) k_smatb_force_mixed(Arena A, Bloc
   const SmF32* tab = smf_table<ONE>(A, S, tab_sh);
   const int i = M.first[blockIdx.x] + threadIdx.x / K;
   double4 F;
-  force_mixed_body<K, ONE, VIR>(A, M, s, S, tab, i, threadIdx.x % K, i < M.end[blockIdx.x], F);
+  force_mixed_body<K, ONE, VIR>(src_arena(A, S, A.st[s]), A, M, s, S, tab, i, threadIdx.x % K, i < M.end[blockIdx.x], F);
 }
 
 // ------------------------------------------------------------------ LJ
@@ -1759,108 +1940,161 @@ __global__ void __launch_bounds__(BLOCK, MINB) k_smatb_force_mixed(Arena A, Bloc
 //   f = -e cos(aux) (pi/2) r / (rc - r1);  r <= r1: p = -e, f = 0
 // wca_interact (src/Pairs.F90:508-589) is LJ with eshift = -e
 // VIR: also the pair virial of the system (virial_close).
-template <int K, bool VIR>
-__global__ void __launch_bounds__(BLOCK) k_lj_fp64(Arena A, BlockMap M) {
-  int s = blk_sys(M);
-  if (s < 0) return;  // padding block of a fixed-capacity map
-  const SysDev& S = A.sys[s];
-  int i = M.first[blockIdx.x] + threadIdx.x / K;
-  int lane = threadIdx.x % K;
-  bool act = i < M.end[blockIdx.x];
+// The constants of one species pair, in a per-block table: the unit ev_ui is
+// folded into e48 and e24.  form -1: no interaction, 0: truncated and shifted
+// (the shift), 1: shifted force (prc, frc), 2: slj, 3: sm1.
+struct LjF64 {
+  double e, e4, e48, e24, sg2, rc, rc2, sh, frc, rs, rs2, sa4, sa8;
+  int form, pad;
+};
+__device__ __forceinline__ LjF64 ljd_load(const PairP& P) {
+  LjF64 c;
+  c.e = P.v[0];
+  c.e4 = 4.0 * P.v[0];
+  c.e48 = 48.0 * P.v[0] * EV_UI;
+  c.e24 = 24.0 * P.v[0] * EV_UI;
+  c.sg2 = P.v[1] * P.v[1];
+  c.rc = P.v[2];
+  c.rc2 = P.v[3];
+  c.form = P.v[0] == 0.0 && P.v[1] == 0.0 ? -1 : P.v[8] == 2.0 ? 3 : P.v[8] != 0.0 ? 2 : P.v[7] != 0.0 ? 1 : 0;
+  c.sh = c.form == 1 ? P.v[4] : c.form == 0 ? P.v[6] : 0.0;
+  c.frc = P.v[5];
+  c.rs = P.v[11];
+  c.rs2 = P.v[11] * P.v[11];
+  c.sa4 = P.v[9];
+  c.sa8 = P.v[10];
+  c.pad = 0;
+  return c;
+}
+// the other pair forms inside their cut-off, from the core's p (less sh) and fr
+__device__ __forceinline__ void lj_other(const LjF64& c, double r2, double& p, double& fr) {
+  if (c.form == 3) {
+    // sm1: the reference's force carries a factor r (Pairs.F90:957)
+    const double dr = sqrt(r2), w = c.rc - c.rs;
+    double f = 0.0;
+    p = -c.e;
+    if (dr > c.rs) {
+      const double aux = PI_D * (dr - (c.rs + c.rc) * 0.5) / w;
+      double sn, cs;
+      sincos(aux, &sn, &cs);
+      p = (0.5 + 0.5 * sn) * c.e - c.e;
+      f = -(cs * (0.5 * PI_D) * dr / w) * c.e;
+    }
+    // f == 0 (inside r1) adds nothing, also for coincident atoms
+    fr = f != 0.0 ? f * EV_UI / dr : 0.0;
+  } else if (c.form == 2) {
+    if (r2 >= c.rs2) {
+      const double dr = sqrt(r2), d = dr - c.rc;
+      const double s4 = d * d * d * d;
+      p = c.sa4 * s4 + c.sa8 * s4 * s4;
+      fr = -(4.0 * c.sa4 * s4 + 8.0 * c.sa8 * s4 * s4) / d * EV_UI / dr;
+    }
+  } else {  // shifted force: sh is prc
+    double rinv;
+    const double dr = sqrt_pos(r2, rinv);
+    p = p - c.frc * (dr - c.rc);
+    fr = fma(c.frc * EV_UI, rinv, fr);
+  }
+}
+
+__device__ __forceinline__ void ljd_table(const Arena& A, const SysDev& S, LjF64* tab) {
+  for (int t = threadIdx.x; t < S.ntypes * S.ntypes; t += BLOCK) tab[t] = ljd_load(A.prm[S.param_off + t]);
+  __syncthreads();
+}
+
+__device__ __forceinline__ double lj_energy(double ep) { return ep * 0.5 * EV_UI; }
+
+// The pass for one thread's lane of atom i; lane 0 returns the force and, in
+// F.w, the pair sum of the energy, and stores both (STORE=false: the caller does).
+template <int K, bool VIR, bool STORE = true, class Src>
+__device__ __forceinline__ void lj_fp64_body(const Src& src, const Arena& A, const BlockMap& M, int s, const SysDev& S,
+                                             const LjF64* tab, int i, int lane, bool act, double4& F) {
   double f0 = 0, f1 = 0, f2 = 0, ep = 0;
   double w[6] = {0, 0, 0, 0, 0, 0};
   if (act) {
-    const double4 xi = A.pos[i];
-    const int ti = A.type[i];
-    const int nn = live_entries(A, S, A.st[s], i, min(A.nn[i], A.lcap));
-    auto gat = [&](int j) { return A.pos[j]; };
-    PAIR_LOOP_BEGIN(double4, gat)
-      const PairP& P = A.prm[S.param_off + ti * S.ntypes + A.type[j]];
-      double e = P.v[0];
-      if (e == 0.0 && P.v[1] == 0.0) continue;
-      double v0, v1, v2;
-      vd_fp64(S, xi, gj[u], v0, v1, v2);
-      double dr = v0 * v0 + v1 * v1 + v2 * v2;
-      if (dr > P.v[3]) continue;
-      dr = sqrt(dr);
-      double p, f;
-      if (P.v[8] == 2.0) {
-        // sm1: the reference's force carries a factor dr (Pairs.F90:957)
-        const double w = P.v[2] - P.v[11];
-        if (dr > P.v[11]) {
-          const double aux = PI_D * (dr - (P.v[11] + P.v[2]) * 0.5) / w;
-          double sn, cs;
-          sincos(aux, &sn, &cs);
-          p = (0.5 + 0.5 * sn) * e - e;
-          f = -(cs * (0.5 * PI_D) * dr / w) * e;
-        } else {
-          p = -e;
-          f = 0.0;
-        }
-      } else if (P.v[8] != 0.0 && dr >= P.v[11]) {
-        const double d = dr - P.v[2];
-        const double s4 = d * d * d * d;
-        p = P.v[9] * s4 + P.v[10] * s4 * s4;
-        f = -(4.0 * P.v[9] * s4 + 8.0 * P.v[10] * s4 * s4) / d;
-      } else {
-        double t = P.v[1] / dr;
-        double t3 = t * t * t;
-        double s6 = t3 * t3;
-        p = P.v[8] != 0.0 ? 4.0 * e * (s6 - 1.0) * s6 : 4.0 * e * (s6 * s6 - s6);
-        f = e * (48.0 * s6 - 24.0) * s6 / dr;
-        if (P.v[7] != 0.0) {
-          p = p - P.v[4] - P.v[5] * (dr - P.v[2]);
-          f = f + P.v[5];
-        } else {
-          p = p - P.v[6];
+    const double4 xi = src.x(i);
+    const bool one = S.ntypes == 1;
+    const LjF64* row = tab + (one ? 0 : src.type(i) * S.ntypes);
+    const ImgTest img = img_test(S);
+    const int nn = src.count(i);
+    auto body = [&](const int (&jj)[UNR], const double4 (&gj)[UNR]) {
+      double v[UNR][3];
+      vd_fp64(S, img, xi, gj, v);
+#pragma unroll
+      for (int u = 0; u < UNR; u++) {
+        const LjF64& c = row[one || jj[u] < 0 ? 0 : src.type(jj[u])];
+        const double r2 = v[u][0] * v[u][0] + v[u][1] * v[u][1] + v[u][2] * v[u][2];
+        const bool off = jj[u] < 0 || c.form < 0 || r2 > c.rc2;
+        // the Lennard-Jones core, branch-free so the group's chains interleave
+        const double ir2 = rcp_pos(off ? 1.0 : r2);
+        const double t2 = c.sg2 * ir2;
+        const double s6 = t2 * t2 * t2;
+        double p = c.e4 * (s6 * s6 - s6) - c.sh;       // the pair energy
+        double fr = (c.e48 * s6 - c.e24) * s6 * ir2;   // f ev_ui / r
+        if (c.form > 0 && !off) lj_other(c, r2, p, fr);
+        if (off) p = fr = 0.0;
+        f0 -= fr * v[u][0];
+        f1 -= fr * v[u][1];
+        f2 -= fr * v[u][2];
+        ep += p;
+        if constexpr (VIR) {
+          const double h = 0.5 * fr;
+          w[0] += h * v[u][0] * v[u][0];
+          w[1] += h * v[u][1] * v[u][1];
+          w[2] += h * v[u][2] * v[u][2];
+          w[3] += h * v[u][0] * v[u][1];
+          w[4] += h * v[u][0] * v[u][2];
+          w[5] += h * v[u][1] * v[u][2];
         }
       }
-      // f == 0 (sm1 inside r1) adds nothing, also for coincident atoms
-      double fr = f != 0.0 ? f * EV_UI / dr : 0.0;
-      f0 -= fr * v0;
-      f1 -= fr * v1;
-      f2 -= fr * v2;
-      ep += p;
-      if constexpr (VIR) {
-        const double h = 0.5 * fr;
-        w[0] += h * v0 * v0;
-        w[1] += h * v1 * v1;
-        w[2] += h * v2 * v2;
-        w[3] += h * v0 * v1;
-        w[4] += h * v0 * v2;
-        w[5] += h * v1 * v2;
-      }
-    PAIR_LOOP_END
+    };
+    pair_groups<K, UNR>(src, i, nn, lane, xi, [&](int j) { return src.x(j); }, body);
   }
   f0 = lane_sum<K>(f0);
   f1 = lane_sum<K>(f1);
   f2 = lane_sum<K>(f2);
   ep = lane_sum<K>(ep);
-  if (act && lane == 0) {
-    A.force[i] = make_double4(f0, f1, f2, 0.0);
-    A.epot[i] = ep * 0.5 * EV_UI;
+  F = make_double4(f0, f1, f2, ep);  // in every lane
+  if constexpr (STORE) {
+    if (act && lane == 0) {
+      A.force[i] = make_double4(f0, f1, f2, 0.0);
+      A.epot[i] = lj_energy(ep);
+    }
   }
   if constexpr (VIR) virial_close(A, M, s, w);
 }
 
+template <int K, bool VIR>
+__global__ void __launch_bounds__(BLOCK) k_lj_fp64(Arena A, BlockMap M) {
+  int s = blk_sys(M);
+  if (s < 0) return;  // padding block of a fixed-capacity map
+  const int i = M.first[blockIdx.x] + threadIdx.x / K;
+  const SysDev& S = A.sys[s];
+  __shared__ LjF64 tab[MAXT * MAXT];
+  ljd_table(A, S, tab);
+  double4 F;
+  lj_fp64_body<K, VIR>(src_arena(A, S, A.st[s]), A, M, s, S, tab, i, threadIdx.x % K, i < M.end[blockIdx.x], F);
+}
+
 // The float constants of one LJ species pair, in a per-block table: 4e,
-// 48e, 24e, sigma^2, rc^2, and by form -- 0: truncated and shifted (the
+// 48 e ev_ui, -24 e ev_ui, sigma^2, rc^2, and by form -- 0: truncated and shifted (the
 // shift), 1: shifted force (prc, frc, rc), 2: slj (rs^2, sa4, sa8, rc).
 struct LjF32 {
-  float e4, e48, e24, sg2, rc2, sh, frc, rc, rs2, sa4, sa8;
+  float e4, e48, ne24, sg2, rc2, nsh, sh, frc, rc, rs2, sa4, sa8;
   int form, on;
 };
 __device__ __forceinline__ LjF32 ljf_load(const PairP& P) {
   LjF32 c;
   const double e = P.v[0], sg = P.v[1];
   c.e4 = (float)(4.0 * e);
-  c.e48 = (float)(48.0 * e);
-  c.e24 = (float)(24.0 * e);
+  c.e48 = (float)(48.0 * e * EV_UI);
+  c.ne24 = (float)(-24.0 * e * EV_UI);
   c.sg2 = (float)(sg * sg);
   c.rc2 = (float)P.v[3];
   c.rc = (float)P.v[2];
   c.form = P.v[8] != 0.0 ? 2 : P.v[7] != 0.0 ? 1 : 0;
-  c.sh = (float)(c.form == 1 ? P.v[4] : P.v[6]);
+  c.sh = (float)(c.form == 1 ? P.v[4] : c.form == 0 ? P.v[6] : 0.0);
+  c.nsh = -c.sh;
   c.frc = (float)P.v[5];
   c.rs2 = (float)(P.v[11] * P.v[11]);
   c.sa4 = (float)P.v[9];
@@ -1869,103 +2103,120 @@ __device__ __forceinline__ LjF32 ljf_load(const PairP& P) {
   return c;
 }
 
+// the other forms inside their cut-off, from the core's p (less sh) and fr
+__device__ __forceinline__ void lj_other(const LjF32& c, float r2, float& p, float& fr) {
+  if (c.form == 2) {
+    // slj (Pairs.F90:403-470): plain LJ inside rs, the quartic-octic
+    // spline sa4 d^4 + sa8 d^8 (d = r - rc) from rs to rc
+    if (r2 >= c.rs2) {
+      const float dr = sqrtf(r2), d = dr - c.rc;
+      const float s4 = d * d * d * d;
+      p = c.sa4 * s4 + c.sa8 * s4 * s4;
+      fr = -(4.0f * c.sa4 * s4 + 8.0f * c.sa8 * s4 * s4) / (d * dr) * (float)EV_UI;
+    }
+  } else {  // shifted force (plj, Pairs.F90:282-370)
+    const float dr = sqrtf(r2);
+    p = p - c.frc * (dr - c.rc);
+    fr = fr + c.frc / dr * (float)EV_UI;
+  }
+}
+__device__ __forceinline__ float rcp_mufu(float x) {
+  float y;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
+}
+
 // Mixed LJ: FP32 pair math from the fixed-point geometry, the species
 // table in shared memory, the FP32 terms of each group of UNR pairs summed
 // and the group sums accumulated per atom in FP64.
+template <int K, bool VIR = false, bool STORE = true, class Src>
+__device__ __forceinline__ void lj_mixed_body(const Src& src, const Arena& A, const BlockMap& M, int s,
+                                              const SysDev& S, const LjF32* tab, int i, int lane, bool act,
+                                              double4& F) {
+  double f0 = 0, f1 = 0, f2_ = 0, ep = 0;
+  double w[6] = {0, 0, 0, 0, 0, 0};
+  if (act) {
+    const int4 xi = src.fx(i);
+    const int nn = src.count(i);
+    const LjF32* row = tab + xi.w * S.ntypes;
+    // one species: its constants stay in registers
+    auto loop = [&](auto one) {
+      const LjF32 c1 = row[0];
+      auto body = [&](const int (&jj)[UNR], const int4 (&gj)[UNR]) {
+        float g0 = 0.0f, g1 = 0.0f, g2 = 0.0f, ge = 0.0f;
+        float gw[6] = {0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f};
+#pragma unroll
+        for (int u = 0; u < UNR; u += 2) {
+          const LjF32& a = one ? c1 : row[gj[u].w];
+          const LjF32& b = one ? c1 : row[gj[u + 1].w];
+          float2 v[3];
+          vd_fx2(S, xi, gj[u], gj[u + 1], v);
+          const float2 r2 = norm2(v);
+          const bool oka = jj[u] >= 0 && !(r2.x > a.rc2) && a.on, okb = jj[u + 1] >= 0 && !(r2.y > b.rc2) && b.on;
+          // 1/r2: the MUFU estimate and a Newton step (within an ulp's rounding)
+          const float2 q2 = f2(oka ? r2.x : a.rc2, okb ? r2.y : b.rc2);
+          float2 ir2 = f2(rcp_mufu(q2.x), rcp_mufu(q2.y));
+          ir2 = fma2(ir2, fma2(q2, ir2 * f2(-1.0f), f2(1.0f)), ir2);
+          const float2 t2 = f2(a.sg2, b.sg2) * ir2;
+          const float2 s6 = t2 * t2 * t2;
+          float2 p = fma2(f2(a.e4, b.e4), fma2(s6, s6, s6 * f2(-1.0f)), f2(a.nsh, b.nsh));
+          float2 fr = fma2(f2(a.e48, b.e48), s6, f2(a.ne24, b.ne24)) * s6 * ir2;  // f ev_ui / r
+          if (oka && a.form > 0) lj_other(a, r2.x, p.x, fr.x);
+          if (okb && b.form > 0) lj_other(b, r2.y, p.y, fr.y);
+          fr = f2(oka ? fr.x : 0.0f, okb ? fr.y : 0.0f);
+          g0 = fmaf(fr.y, v[0].y, fmaf(fr.x, v[0].x, g0));
+          g1 = fmaf(fr.y, v[1].y, fmaf(fr.x, v[1].x, g1));
+          g2 = fmaf(fr.y, v[2].y, fmaf(fr.x, v[2].x, g2));
+          ge += oka ? p.x : 0.0f;
+          ge += okb ? p.y : 0.0f;
+          if constexpr (VIR) {
+            const float2 h = fr * f2(0.5f);
+            const float2 hx = h * v[0], hy = h * v[1], hz = h * v[2];
+            const float2 q[6] = {hx * v[0], hy * v[1], hz * v[2], hx * v[1], hx * v[2], hy * v[2]};
+            for (int k = 0; k < 6; k++) gw[k] += q[k].x + q[k].y;
+          }
+        }
+        f0 -= (double)g0;
+        f1 -= (double)g1;
+        f2_ -= (double)g2;
+        ep += (double)ge;
+        if constexpr (VIR)
+          for (int k = 0; k < 6; k++) w[k] += (double)gw[k];
+      };
+      pair_groups<K, UNR>(src, i, nn, lane, xi, [&](int j) { return src.fx(j); }, body);
+    };
+    if (S.ntypes == 1) loop(std::true_type{});
+    else loop(std::false_type{});
+  }
+  f0 = lane_sum<K>(f0);
+  f1 = lane_sum<K>(f1);
+  f2_ = lane_sum<K>(f2_);
+  ep = lane_sum<K>(ep);
+  F = make_double4(f0, f1, f2_, ep);  // in every lane
+  if constexpr (STORE) {
+    if (act && lane == 0) {
+      A.force[i] = make_double4(f0, f1, f2_, 0.0);
+      A.epot[i] = lj_energy(ep);
+    }
+  }
+  if constexpr (VIR) virial_close(A, M, s, w);
+}
+
+__device__ __forceinline__ void ljf_table(const Arena& A, const SysDev& S, LjF32* tab) {
+  for (int t = threadIdx.x; t < S.ntypes * S.ntypes; t += BLOCK) tab[t] = ljf_load(A.prm[S.param_off + t]);
+  __syncthreads();
+}
+
 template <int K, bool VIR = false>
 __global__ void __launch_bounds__(BLOCK) k_lj_mixed(Arena A, BlockMap M) {
   int s = blk_sys(M);
   if (s < 0) return;  // padding block of a fixed-capacity map
   const SysDev& S = A.sys[s];
   __shared__ LjF32 tab[MAXT * MAXT];
-  for (int t = threadIdx.x; t < S.ntypes * S.ntypes; t += BLOCK) tab[t] = ljf_load(A.prm[S.param_off + t]);
-  __syncthreads();
-  int i = M.first[blockIdx.x] + threadIdx.x / K;
-  int lane = threadIdx.x % K;
-  bool act = i < M.end[blockIdx.x];
-  double f0 = 0, f1 = 0, f2 = 0, ep = 0;
-  double w[6] = {0, 0, 0, 0, 0, 0};
-  if (act) {
-    const int4 xi = A.fxp[i];
-    const int nn = live_entries(A, S, A.st[s], i, min(A.nn[i], A.lcap));
-    const float evui = (float)EV_UI;
-    const LjF32* row = tab + xi.w * S.ntypes;
-    int jn[UNR];
-    list_group<K>(A, i, nn, lane, jn);
-    for (int m0 = lane; m0 < nn; m0 += UNR * K) {
-      int jj[UNR];
-#pragma unroll
-      for (int u = 0; u < UNR; u++) jj[u] = jn[u];
-      int4 gj[UNR];
-#pragma unroll
-      for (int u = 0; u < UNR; u++) {
-        gj[u] = xi;  // an empty slot: a zero pair vector, masked below
-        if (jj[u] >= 0) gj[u] = A.fxp[jj[u]];
-      }
-      list_group<K>(A, i, nn, m0 + UNR * K, jn);  // next group's ids, in flight meanwhile
-      float g0 = 0.0f, g1 = 0.0f, g2 = 0.0f, ge = 0.0f;
-      float gw[6] = {0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f};
-#pragma unroll
-      for (int u = 0; u < UNR; u++) {
-        const int4 xj = gj[u];
-        const LjF32& c = row[xj.w];
-        float v0, v1, v2;
-        vd_fx(S, xi, xj, v0, v1, v2);
-        const float r2 = v0 * v0 + v1 * v1 + v2 * v2;
-        const bool ok = jj[u] >= 0 && !(r2 > c.rc2) && c.on;
-        const float ir2 = __frcp_rn(ok ? r2 : c.rc2);
-        const float t2 = c.sg2 * ir2;
-        const float s6 = t2 * t2 * t2;
-        float p = c.e4 * (s6 * s6 - s6);
-        float fr = (c.e48 * s6 - c.e24) * s6 * ir2;  // f / r
-        if (c.form == 2) {
-          // slj (Pairs.F90:403-470): plain LJ inside rs, the quartic-octic
-          // spline sa4 d^4 + sa8 d^8 (d = r - rc) from rs to rc
-          if (ok && r2 >= c.rs2) {
-            const float dr = sqrtf(r2), d = dr - c.rc;
-            const float s4 = d * d * d * d;
-            p = c.sa4 * s4 + c.sa8 * s4 * s4;
-            fr = -(4.0f * c.sa4 * s4 + 8.0f * c.sa8 * s4 * s4) / (d * dr);
-          }
-        } else if (c.form == 1) {  // shifted force (plj, Pairs.F90:282-370)
-          const float dr = sqrtf(ok ? r2 : c.rc2);
-          p = p - c.sh - c.frc * (dr - c.rc);
-          fr = fr + c.frc / dr;
-        } else {
-          p = p - c.sh;
-        }
-        fr = ok ? fr * evui : 0.0f;
-        g0 = fmaf(fr, v0, g0);
-        g1 = fmaf(fr, v1, g1);
-        g2 = fmaf(fr, v2, g2);
-        ge += ok ? p : 0.0f;
-        if constexpr (VIR) {
-          const float h = 0.5f * fr;
-          gw[0] += h * v0 * v0;
-          gw[1] += h * v1 * v1;
-          gw[2] += h * v2 * v2;
-          gw[3] += h * v0 * v1;
-          gw[4] += h * v0 * v2;
-          gw[5] += h * v1 * v2;
-        }
-      }
-      f0 -= (double)g0;
-      f1 -= (double)g1;
-      f2 -= (double)g2;
-      ep += (double)ge;
-      if constexpr (VIR)
-        for (int k = 0; k < 6; k++) w[k] += (double)gw[k];
-    }
-  }
-  f0 = lane_sum<K>(f0);
-  f1 = lane_sum<K>(f1);
-  f2 = lane_sum<K>(f2);
-  ep = lane_sum<K>(ep);
-  if (act && lane == 0) {
-    A.force[i] = make_double4(f0, f1, f2, 0.0);
-    A.epot[i] = ep * 0.5 * EV_UI;
-  }
-  if constexpr (VIR) virial_close(A, M, s, w);
+  ljf_table(A, S, tab);
+  const int i = M.first[blockIdx.x] + threadIdx.x / K;
+  double4 F;
+  lj_mixed_body<K, VIR>(src_arena(A, S, A.st[s]), A, M, s, S, tab, i, threadIdx.x % K, i < M.end[blockIdx.x], F);
 }
 
 // ------------------------------------------------------------------ Tersoff
@@ -2015,15 +2266,18 @@ __device__ __forceinline__ R ts_fc(R r, R r1, R r2, R& dfc) {
   return R(0.5) - R(0.5) * sn;
 }
 
+__device__ __forceinline__ float ts_rcp(float a) { return 1.0f / a; }
+__device__ __forceinline__ double ts_rcp(double a) { return rcp_pos(a); }
+
 // bond order of one bond: b, b VA (FP64) and db/dzeta
 __device__ __forceinline__ void ts_border(const TersoffP& T, double z, double va, double& b, double& bva,
                                           double& dbdz) {
   if (z > 1.0e-15) {
-    const double zn = pow(z, T.n);
-    const double x = pow(T.beta, T.n) * zn;
-    const double aux = 1.0 / (1.0 + x);
-    b = T.chi * pow(aux, 0.5 / T.n);
-    dbdz = -0.5 * b * aux * x / z;
+    // x = (beta z)^n and (1 + x)^(-1/2n) through exp and log (of the sum's
+    // logarithms: two functions each instead of the general power's cases)
+    const double x = exp(T.n * log(T.beta * z));
+    b = T.chi * exp(-0.5 / T.n * log1p(x));
+    dbdz = -0.5 * b * x / ((1.0 + x) * z);
   } else {
     b = T.chi;
     dbdz = 0.0;
@@ -2059,14 +2313,15 @@ __host__ __device__ constexpr size_t tsf_smem() {
   return (size_t)8 * (BLOCK / TPA) * TS_MAXB * sizeof(R);  // eight per-bond arrays
 }
 
-template <typename R, int MINB, int TPA>
-__global__ void __launch_bounds__(BLOCK, MINB) k_tsf_bonds(Arena A, BlockMap M) {
+// The bond pass over the BLOCK / TPA atoms from `first` (up to `end`), by the whole block.
+template <typename R, int TPA>
+__device__ __forceinline__ void tsf_bonds_body(const Arena& A, int s, const SysDev& S, int lk, int first, int end,
+                                               unsigned char* tsf_sh) {
   constexpr int APB = BLOCK / TPA;
   constexpr int NB = APB * TS_MAXB;
   constexpr bool MIXED = sizeof(R) == 4;
   constexpr int PER = TS_MAXB / TPA;  // bonds per thread at most
   constexpr int CH = TPA == 2 ? 2 : 1;  // bonds a thread carries at once
-  extern __shared__ __align__(16) unsigned char tsf_sh[];
   R* sux = reinterpret_cast<R*>(tsf_sh);
   R* suy = sux + NB;
   R* suz = suy + NB;
@@ -2075,17 +2330,14 @@ __global__ void __launch_bounds__(BLOCK, MINB) k_tsf_bonds(Arena A, BlockMap M) 
   R* sdfc = sfc + NB;
   R* spre = sdfc + NB;
   R* sdv = spre + NB;  // the radial pair derivative dV of each bond (its owner's)
-  const int s = blk_sys(M);
-  if (s < 0) return;  // padding block of a fixed-capacity map
-  const SysDev& S = A.sys[s];
   const TersoffP& T = S.ts;
   const unsigned FULL = 0xffffffffu;
   const int lane = threadIdx.x & 31, q = threadIdx.x & (TPA - 1), la = threadIdx.x / TPA;
-  const int i = M.first[blockIdx.x] + la;
-  const bool act = i < M.end[blockIdx.x];
+  const int i = first + la;
+  const bool act = i < end;
   const int base = la * TS_MAXB;
   const double r1 = T.R - T.D, r2 = T.R + T.D;
-  const int nl = act ? live_entries(A, S, A.st[s], i, min(A.nn[i], A.lcap)) : 0;
+  const int nl = act ? live_entries<false>(A, lk, i, min(A.nn[i], A.lcap)) : 0;
 
   // ---- bonds in flist order: the atom's TPA threads test TPA slots at a
   // time and a ballot ranks the bonds they found
@@ -2095,6 +2347,7 @@ __global__ void __launch_bounds__(BLOCK, MINB) k_tsf_bonds(Arena A, BlockMap M) 
     if constexpr (MIXED) qi = A.fxp[i];
     else xi = A.pos[i];
   }
+  const ImgTest img = img_test(S);
   int cnt = 0, err = 0;
   unsigned long long mask = 0ull;
   const int tmax = __reduce_max_sync(FULL, (nl + TPA - 1) / TPA);
@@ -2130,10 +2383,11 @@ __global__ void __launch_bounds__(BLOCK, MINB) k_tsf_bonds(Arena A, BlockMap M) 
             u0 = v0 * ir; u1 = v1 * ir; u2 = v2 * ir;
             bond = rr <= (float)r2;
           } else {
-            double v0, v1, v2;
-            vd_fp64(S, xi, xj[u], v0, v1, v2);
-            rr = sqrt(v0 * v0 + v1 * v1 + v2 * v2);
-            u0 = v0 / rr; u1 = v1 / rr; u2 = v2 / rr;
+            const double4 one[1] = {xj[u]};
+            double v[1][3], ir;
+            vd_fp64(S, img, xi, one, v);
+            rr = sqrt_pos(v[0][0] * v[0][0] + v[0][1] * v[0][1] + v[0][2] * v[0][2], ir);
+            u0 = v[0][0] * ir; u1 = v[0][1] * ir; u2 = v[0][2] * ir;
             bond = !(rr > r2);
           }
         }
@@ -2186,7 +2440,7 @@ __global__ void __launch_bounds__(BLOCK, MINB) k_tsf_bonds(Arena A, BlockMap M) 
         if (b == (e ? a1 : a0) || (e == 1 && !h1)) continue;
         const R ct = ax[e] * bx + ay[e] * by + az[e] * bz;
         const R hc = h - ct, hq = hc * hc;
-        z[e] += fcb * (R(1) + c2d2 * hq / (d2 + hq));  // 1 + c2/d2 - c2/(d2+hc2), no cancellation
+        z[e] += fcb * (R(1) + c2d2 * hq * ts_rcp(d2 + hq));  // 1 + c2/d2 - c2/(d2+hc2), no cancellation
       }
     }
 #pragma unroll
@@ -2224,7 +2478,7 @@ __global__ void __launch_bounds__(BLOCK, MINB) k_tsf_bonds(Arena A, BlockMap M) 
       const int a = e ? k1 : a0;
       ax[e] = sux[base + a]; ay[e] = suy[base + a]; az[e] = suz[base + a];
       fca[e] = sfc[base + a]; dfca[e] = sdfc[base + a]; pa[e] = spre[base + a];
-      ira[e] = R(1) / sr[base + a];
+      ira[e] = ts_rcp(sr[base + a]);
       tx[e] = ty[e] = tz[e] = R(0);
     }
     for (int b = 0; b < nb; b++) {
@@ -2234,7 +2488,7 @@ __global__ void __launch_bounds__(BLOCK, MINB) k_tsf_bonds(Arena A, BlockMap M) 
       for (int e = 0; e < CH; e++) {
         if (b == (e ? a1 : a0) || (e == 1 && !h1)) continue;
         const R ct = ax[e] * bx + ay[e] * by + az[e] * bz;
-        const R hc = h - ct, iden = R(1) / (d2 + hc * hc);
+        const R hc = h - ct, iden = ts_rcp(d2 + hc * hc);
         const R g = R(1) + c2d2 * (hc * hc) * iden;
         const R dg = R(-2) * c2 * hc * iden * iden;  // dg / dcos
         const R coef = (pa[e] * fcb + pb * fca[e]) * dg * ira[e];
@@ -2284,13 +2538,17 @@ __global__ void __launch_bounds__(BLOCK, MINB) k_tsf_bonds(Arena A, BlockMap M) 
   if (act && err) atomicOr(&A.st[s].status, ST_BONDS);
 }
 
+template <typename R, int MINB, int TPA>
+__global__ void __launch_bounds__(BLOCK, MINB) k_tsf_bonds(Arena A, BlockMap M) {
+  extern __shared__ __align__(16) unsigned char tsf_sh[];
+  const int s = blk_sys(M);
+  if (s < 0) return;  // padding block of a fixed-capacity map
+  tsf_bonds_body<R, TPA>(A, s, A.sys[s], live_band(A.sys[s], A.st[s]), M.first[blockIdx.x], M.end[blockIdx.x], tsf_sh);
+}
+
 // F_l += the bond records of l's partners for their bonds to l (slot order)
 template <typename R>
-__global__ void __launch_bounds__(BLOCK / 2) k_tsf_gather(Arena A, BlockMap M) {
-  const int s = blk_sys(M);
-  if (s < 0) return;
-  const int i = M.first[blockIdx.x] + threadIdx.x;
-  if (i >= M.end[blockIdx.x]) return;
+__device__ __forceinline__ double4 tsf_gather_body(const Arena& A, int s, int i) {
   unsigned long long mk = A.tsmask[i];
   double4 f = A.force[i];
   bool bad = false;
@@ -2316,38 +2574,50 @@ __global__ void __launch_bounds__(BLOCK / 2) k_tsf_gather(Arena A, BlockMap M) {
       f.z += b.z;
     }
   }
-  A.force[i] = f;
   if (bad) atomicOr(&A.st[s].status, ST_BONDS);
+  return f;
 }
 
-// reverse slots of the Tersoff systems flagged for a rebuild: for each list
-// entry (i, m) with partner j, the slot of i in j's flist (255: none)
+template <typename R>
+__global__ void __launch_bounds__(BLOCK / 2) k_tsf_gather(Arena A, BlockMap M) {
+  const int s = blk_sys(M);
+  if (s < 0) return;
+  const int i = M.first[blockIdx.x] + threadIdx.x;
+  if (i < M.end[blockIdx.x]) A.force[i] = tsf_gather_body<R>(A, s, i);
+}
+
+// reverse slots: for each list entry (i, m) with partner j, the slot of i in
+// j's flist (255: none); entries m0, m0 + dm, ... of atom i
+__device__ __forceinline__ void tsf_rslot_row(const Arena& A, int i, int m0, int dm) {
+  const int n = min(A.nn[i], A.lcap);
+  for (int m = m0; m < n; m += dm) {
+    const size_t e = (size_t)m * A.cap + i;
+    const int j = A.flist[e];
+    int r = 255;
+    if ((unsigned)j < (unsigned)A.cap) {
+      const int nj = min(min(A.nn[j], A.lcap), 255);
+      // the first slot of j's list that holds i, four loads in flight at a time
+      for (int k0 = 0; k0 < nj && r == 255; k0 += 4) {
+        int v[4];
+#pragma unroll
+        for (int u = 0; u < 4; u++) v[u] = k0 + u < nj ? A.flist[(size_t)(k0 + u) * A.cap + j] : -1;
+#pragma unroll
+        for (int u = 3; u >= 0; u--)
+          if (v[u] == i) r = k0 + u;
+      }
+    }
+    A.rslot[e] = (unsigned char)r;
+  }
+}
+
+// the reverse slots of the Tersoff systems flagged for a rebuild
 __global__ void k_tsf_rslot(Arena A, BlockMap M) {
   rebuild_items(M.nblk, [&](int b) {
       const int s = M.sys[b];
       return s >= 0 && A.st[s].rebuild && A.sys[s].ff == FF_TERSOFF;
     }, [&](int b) {
       const int i = M.first[b] + threadIdx.x;
-      if (i >= M.end[b]) return;
-      const int n = min(A.nn[i], A.lcap);
-      for (int m = 0; m < n; m++) {
-        const size_t e = (size_t)m * A.cap + i;
-        const int j = A.flist[e];
-        int r = 255;
-        if ((unsigned)j < (unsigned)A.cap) {
-          const int nj = min(min(A.nn[j], A.lcap), 255);
-          // the first slot of j's list that holds i, four loads in flight at a time
-          for (int k0 = 0; k0 < nj && r == 255; k0 += 4) {
-            int v[4];
-#pragma unroll
-            for (int u = 0; u < 4; u++) v[u] = k0 + u < nj ? A.flist[(size_t)(k0 + u) * A.cap + j] : -1;
-#pragma unroll
-            for (int u = 3; u >= 0; u--)
-              if (v[u] == i) r = k0 + u;
-          }
-        }
-        A.rslot[e] = (unsigned char)r;
-      }
+      if (i < M.end[b]) tsf_rslot_row(A, i, 0, 1);
     });
 }
 
@@ -2386,35 +2656,48 @@ __global__ void k_zero_force(Arena A, BlockMap M) {
 // ------------------------------------------------------------------ integrators
 // ---- per-atom integrator updates, shared by the split and fused kernels
 // velocity_verlet_b (src/Integration.F90:1171-1186)
-__device__ __forceinline__ void vv_b_atom(double dt, double om, const double4& F, double4& v, double4& a) {
+__device__ __forceinline__ void vv_b_c(double dt, double om, double F, double& v, double& a) {
   const double adv = dt * 0.5;
-  a.x = F.x * om; a.y = F.y * om; a.z = F.z * om;
-  v.x = v.x + adv * a.x;
-  v.y = v.y + adv * a.y;
-  v.z = v.z + adv * a.z;
+  a = F * om;
+  v = v + adv * a;
+}
+__device__ __forceinline__ void vv_b_atom(double dt, double om, const double4& F, double4& v, double4& a) {
+  vv_b_c(dt, om, F.x, v.x, a.x);
+  vv_b_c(dt, om, F.y, v.y, a.y);
+  vv_b_c(dt, om, F.z, v.z, a.z);
 }
 
 // ermak_b (src/Integration.F90:1013-1031)
+// in two parts: w = cc0 v + (cc1 - cc2) a + vv holds all that is known before
+// the force, so between two steps of a captured chunk an atom carries w in
+// its velocity slot instead of v, a and vv (96 B of 256 less per step), and
+// v = w + cc2 F/m.  Explicit fused multiply-adds: every path rounds alike.
+__device__ __forceinline__ double ermak_w(const SysDev& S, double v, double a, double vv) {
+  return __fma_rn(S.cc0, v, __fma_rn(S.cc1 - S.cc2, a, vv));
+}
+__device__ __forceinline__ double ermak_v(const SysDev& S, double om, double F, double w) {
+  return __fma_rn(__dmul_rn(S.cc2, om), F, w);
+}
 __device__ __forceinline__ void ermak_b_atom(const SysDev& S, double om, const double4& F, const double4& vv,
                                              double4& v, double4& a) {
-  const double c12 = S.cc1 - S.cc2;
-  v.x = S.cc0 * v.x + c12 * a.x + S.cc2 * F.x * om + vv.x;
-  v.y = S.cc0 * v.y + c12 * a.y + S.cc2 * F.y * om + vv.y;
-  v.z = S.cc0 * v.z + c12 * a.z + S.cc2 * F.z * om + vv.z;
+  v.x = ermak_v(S, om, F.x, ermak_w(S, v.x, a.x, vv.x));
+  v.y = ermak_v(S, om, F.y, ermak_w(S, v.y, a.y, vv.y));
+  v.z = ermak_v(S, om, F.z, ermak_w(S, v.z, a.z, vv.z));
   a.x = F.x * om; a.y = F.y * om; a.z = F.z * om;
 }
 
 // velocity_verlet_a (src/Integration.F90:1150-1168)
+__device__ __forceinline__ void vv_a_c(double dt, double om, double F, double& x, double& v, double& a) {
+  const double adv = dt * 0.5, adx = adv * dt;
+  a = F * om;
+  x = x + dt * v + adx * a;
+  v = v + adv * a;
+}
 __device__ __forceinline__ void vv_a_atom(double dt, double om, const double4& F, double4& x, double4& v,
                                           double4& a) {
-  const double adv = dt * 0.5, adx = adv * dt;
-  a.x = F.x * om; a.y = F.y * om; a.z = F.z * om;
-  x.x = x.x + dt * v.x + adx * a.x;
-  x.y = x.y + dt * v.y + adx * a.y;
-  x.z = x.z + dt * v.z + adx * a.z;
-  v.x = v.x + adv * a.x;
-  v.y = v.y + adv * a.y;
-  v.z = v.z + adv * a.z;
+  vv_a_c(dt, om, F.x, x.x, v.x, a.x);
+  vv_a_c(dt, om, F.y, x.y, v.y, a.y);
+  vv_a_c(dt, om, F.z, x.z, v.z, a.z);
 }
 
 // nordsieck_predictor (src/Integration.F90:1192-1228): the fifth-order Gear
@@ -2433,7 +2716,7 @@ __device__ __forceinline__ double nord_pred(double dt, double& x, double& v, dou
   return x;
 }
 
-__device__ __forceinline__ void nord_a_atom(Arena& A, double dt, int i, double4& x, double4& v, double4& a) {
+__device__ __forceinline__ void nord_a_atom(const Arena& A, double dt, int i, double4& x, double4& v, double4& a) {
   double4 a2 = A.acel2[i], a3 = A.acel3[i];
   const double4 a4 = A.acel4[i];
   nord_pred(dt, x.x, v.x, a.x, a2.x, a3.x, a4.x);
@@ -2458,7 +2741,7 @@ __device__ __forceinline__ void nord_corr(double dt, double hm, double F, double
   v = v / dt;
 }
 
-__device__ __forceinline__ void nord_b_atom(Arena& A, double dt, double om, int i, const double4& F, double4& x,
+__device__ __forceinline__ void nord_b_atom(const Arena& A, double dt, double om, int i, const double4& F, double4& x,
                                             double4& v, double4& a) {
   double4 a2 = A.acel2[i], a3 = A.acel3[i], a4 = A.acel4[i];
   const double hm = dt * dt / 2.0 * om;
@@ -2471,7 +2754,15 @@ __device__ __forceinline__ void nord_b_atom(Arena& A, double dt, double om, int 
 }
 
 // ermak_a (src/Integration.F90:963-1011): position update and the velocity
-// kick vel_v that ermak_b adds
+// kick vel_v that ermak_b adds (..._c: one coordinate, the same operations)
+__device__ __forceinline__ void ermak_a_c(const SysDev& S, double2 mi, double r0, double r1, double v, double a,
+                                          double& x, double& vv) {
+  const double f_lan = S.skt * mi.y;
+  const double pr = f_lan * S.sdr, pv = f_lan * S.sdv;
+  vv = pv * (S.crv1 * r0 + S.crv2 * r1);
+  const double c2dt = S.cc2 * S.dt;
+  x = x + S.cc1 * v + c2dt * a + pr * r0;
+}
 __device__ __forceinline__ void ermak_a_atom(const Arena& A, const SysDev& S, const SysState& st, int i,
                                              double2 mi, const double4& v, const double4& a, double4& x,
                                              double4& vv) {
@@ -2495,6 +2786,12 @@ __device__ __forceinline__ void ermak_a_atom(const Arena& A, const SysDev& S, co
 }
 
 // do_pbc_1 (src/Set_Properties.f90:444-470): a single wrap into [0, box)
+__device__ __forceinline__ void wrap_c(const SysDev& S, int c, double& x) {
+  if (S.boxed && S.pbc[c]) {
+    if (x >= S.L[c]) x = x - S.L[c];
+    else if (x < 0.0) x = x + S.L[c];
+  }
+}
 __device__ __forceinline__ void wrap_atom(const SysDev& S, double4& x) {
   if (S.boxed) {
     if (S.pbc[0]) { if (x.x >= S.L[0]) x.x = x.x - S.L[0]; else if (x.x < 0.0) x.x = x.x + S.L[0]; }
@@ -2699,7 +2996,7 @@ __device__ __forceinline__ void axes_sys(SysDev& S, SysState& st) {
 // ------------------------------------------------------------------ LKD
 // Block sums of three per-atom values; true in thread 0 of the system's
 // last block, which then holds the system's totals (added in block order).
-__device__ __forceinline__ bool sys3_close(Arena& A, const BlockMap& M, int s, const double w[3], double t[3]) {
+__device__ __forceinline__ bool sys3_close(const Arena& A, const BlockMap& M, int s, const double w[3], double t[3]) {
   double b[3];
 #pragma unroll
   for (int k = 0; k < 3; k++) b[k] = block_sum(w[k]);
@@ -2867,12 +3164,13 @@ __global__ void k_lgf_sys(Arena A, const int* sys, int nsys) {
 
 // the moved atom's outputs: position, fixed-point copy, skin displacement
 // (xo = its position at the last rebuild, ty = its species)
-__device__ __forceinline__ double moved_atom(Arena& A, const SysDev& S, SysState& st, int i, const double4& x,
-                                             const double4& xo, int ty) {
+// (fxp: where the fixed-point copy goes)
+__device__ __forceinline__ double moved_atom(const Arena& A, const SysDev& S, SysState& st, int i, const double4& x,
+                                             const double4& xo, int ty, int4* fxp) {
   A.pos[i] = x;
   if (S.prec == PREC_MIXED || S.ff == FF_TERSOFF) {
     int bad = 0;
-    write_fx(A, S, i, x, ty, bad);
+    write_fx(fxp, S, i, x, ty, bad);
     if (bad) atomicOr(&st.status, ST_LOST);
   }
   double d = disp2(S, x, xo);
@@ -2886,7 +3184,7 @@ __device__ __forceinline__ double moved_atom(Arena& A, const SysDev& S, SysState
 // the step's integrator bookkeeping.
 // PISTON=false: a kernel that never sees a constant-pressure system
 template <bool COND, bool PISTON = true>
-__device__ __forceinline__ void skin_close(Arena& A, const BlockMap& M, int s, const SysDev& S, SysState& st,
+__device__ __forceinline__ void skin_close(const Arena& A, const BlockMap& M, int s, const SysDev& S, SysState& st,
                                            bool frozen, double2 t, cudaGraphConditionalHandle cond) {
   t = block_top2(t);
   if (threadIdx.x == 0) A.blk_top2[M.base + blockIdx.x] = t;
@@ -2926,7 +3224,9 @@ __device__ __forceinline__ void skin_close(Arena& A, const BlockMap& M, int s, c
 // rebuild raises it, so steps without a rebuild skip those launches.
 // COND=false builds a copy without the device-side graph call, for plain
 // launches (profilers do not replay kernels that contain it).
-template <bool COND>
+// W: the first half step of a chunk of fused steps, after which Ermak atoms
+// carry w in the velocity slot.
+template <bool COND, bool W = false>
 __global__ void __launch_bounds__(BLOCK) k_step_a(Arena A, BlockMap M, cudaGraphConditionalHandle cond) {
   int s = blk_sys(M);
   if (s < 0) return;  // padding block of a fixed-capacity map
@@ -2948,7 +3248,10 @@ __global__ void __launch_bounds__(BLOCK) k_step_a(Arena A, BlockMap M, cudaGraph
     } else if (S.integ == IT_ERMAK) {
       double4 vv;
       ermak_a_atom(A, S, st, i, mi, v, a, x, vv);
-      A.vel_v[i] = vv;
+      if (W)
+        A.vel[i] = make_double4(ermak_w(S, v.x, a.x, vv.x), ermak_w(S, v.y, a.y, vv.y), ermak_w(S, v.z, a.z, vv.z), 0.0);
+      else
+        A.vel_v[i] = vv;
     } else if (S.integ == IT_LGF) {
       double4 pv;
       lgf_a_atom(A, S, st, i, mi.x, A.force[i], v, a, x, pv);
@@ -2979,7 +3282,7 @@ __global__ void __launch_bounds__(BLOCK) k_step_a(Arena A, BlockMap M, cudaGraph
       A.vel[i] = v;
     }
     wrap_atom(S, x);
-    t.x = moved_atom(A, S, st, i, x, A.pos_old[i], A.type[i]);
+    t.x = moved_atom(A, S, st, i, x, A.pos_old[i], A.type[i], A.fxp);
   }
   skin_close<COND>(A, M, s, S, st, frozen, t, cond);
 }
@@ -2989,49 +3292,78 @@ __global__ void __launch_bounds__(BLOCK) k_step_a(Arena A, BlockMap M, cudaGraph
 // registers: the operations of k_step_b and k_step_a in their order.
 // ba_store writes the result.
 struct BaAtom {
-  double4 x, v, a, vv;
+  double4 x, v;  // v: Ermak's w (ermak_w) between the steps of a chunk
   double d;  // squared displacement since the list build (1e-16: not moved)
   int ty;
   bool on;   // velocity Verlet or Ermak
 };
 
-__device__ __forceinline__ void ba_calc(const Arena& A, const SysDev& S, const SysState& st, int i, const double4& F,
-                                        BaAtom& b) {
+// where an atom's integrator state lives: the arena itself, or its
+// shared-memory namesakes
+struct StateRef {
+  double4 *pos, *vel, *acel, *pos_old;
+  double2* minv;
+  int* type;
+};
+
+// (q: the atom's index in X; i: in the arena)
+template <class State>
+__device__ __forceinline__ void ba_calc(const Arena& A, const State& X, int q, const SysDev& S, const SysState& st,
+                                        int i, const double4& F, BaAtom& b) {
   const int integ = S.integ;
   b.on = integ == IT_VV || integ == IT_ERMAK;
   b.d = 1.e-16;
   if (!b.on) return;
   // every input is loaded before the first use, so all loads are in flight together
-  b.x = A.pos[i];
-  b.v = A.vel[i];
-  b.a = A.acel[i];
-  const double2 mi = A.minv[i];
-  const double4 xo = A.pos_old[i];
-  b.ty = A.type[i];
-  const double4 vv0 = integ == IT_ERMAK ? A.vel_v[i] : make_double4(0, 0, 0, 0);
+  b.x = X.pos[q];
+  b.v = X.vel[q];
+  const double2 mi = X.minv[q];
+  const double4 xo = X.pos_old[q];
+  b.ty = X.type[q];
+  double4 a;
   if (integ == IT_VV) {
-    vv_b_atom(S.dt, mi.x, F, b.v, b.a);
-    vv_a_atom(S.dt, mi.x, F, b.x, b.v, b.a);
+    vv_b_atom(S.dt, mi.x, F, b.v, a);
+    vv_a_atom(S.dt, mi.x, F, b.x, b.v, a);
   } else {
-    ermak_b_atom(S, mi.x, F, vv0, b.v, b.a);
-    ermak_a_atom(A, S, st, i, mi, b.v, b.a, b.x, b.vv);
+    b.v.x = ermak_v(S, mi.x, F.x, b.v.x);
+    b.v.y = ermak_v(S, mi.x, F.y, b.v.y);
+    b.v.z = ermak_v(S, mi.x, F.z, b.v.z);
+    a.x = F.x * mi.x; a.y = F.y * mi.x; a.z = F.z * mi.x;
+    double4 vv;
+    ermak_a_atom(A, S, st, i, mi, b.v, a, b.x, vv);
+    b.v.x = ermak_w(S, b.v.x, a.x, vv.x);
+    b.v.y = ermak_w(S, b.v.y, a.y, vv.y);
+    b.v.z = ermak_w(S, b.v.z, a.z, vv.z);
   }
   wrap_atom(S, b.x);
   b.d = disp2(S, b.x, xo);
 }
 
-__device__ __forceinline__ void ba_store(Arena& A, const SysDev& S, SysState& st, int i, const BaAtom& b) {
-  if (!b.on) return;
-  if (S.integ == IT_ERMAK) A.vel_v[i] = b.vv;
-  A.acel[i] = b.a;
-  A.vel[i] = b.v;
-  A.pos[i] = b.x;
+// stores the moved atom's state
+template <class State>
+__device__ __forceinline__ void ba_store(const State& X, int q, SysState& st, const BaAtom& b) {
+  X.vel[q] = b.v;
+  X.pos[q] = b.x;
+  if (!(b.d == b.d)) atomicOr(&st.status, ST_NAN);
+}
+
+// the fixed-point record of a moved atom, where its system keeps one
+__device__ __forceinline__ void ba_fx(const SysDev& S, SysState& st, int i, const BaAtom& b, int4* fxp) {
   if (S.prec == PREC_MIXED || S.ff == FF_TERSOFF) {
     int bad = 0;
-    write_fx(A, S, i, b.x, b.ty, bad);
+    write_fx(fxp, S, i, b.x, b.ty, bad);
     if (bad) atomicOr(&st.status, ST_LOST);
   }
-  if (!(b.d == b.d)) atomicOr(&st.status, ST_NAN);
+}
+
+__device__ __forceinline__ void ba_step(const Arena& A, const SysDev& S, SysState& st, int i, const double4& F,
+                                        double2& t) {
+  BaAtom b;
+  ba_calc(A, A, i, S, st, i, F, b);
+  t = top2_merge(t, make_double2(b.d, 1.e-16));
+  if (!b.on) return;
+  ba_store(A, i, st, b);
+  ba_fx(S, st, i, b, A.fxp);
 }
 
 // step_b of one step fused with step_a of the next, for velocity Verlet and
@@ -3052,13 +3384,7 @@ __global__ void __launch_bounds__(BLOCK, 4) k_step_ba(Arena A, BlockMap M, cudaG
 #pragma unroll 1
   for (int k = 0; k < APT; k++) {
     const int i = M.first[blockIdx.x] + threadIdx.x + k * BLOCK;
-    if (i < M.end[blockIdx.x]) {
-      BaAtom b;
-      b.on = false;
-      ba_calc(A, S, st, i, A.force[i], b);
-      t = top2_merge(t, make_double2(b.d, 1.e-16));
-      ba_store(A, S, st, i, b);
-    }
+    if (i < M.end[blockIdx.x]) ba_step(A, S, st, i, A.force[i], t);
   }
   skin_close<COND, false>(A, M, s, S, st, false, t, cond);
 }
@@ -3083,16 +3409,11 @@ __global__ void __launch_bounds__(BLOCK, MINB) k_smatb_force_mixed_ba(Arena A, B
   const int lane = threadIdx.x % K;
   const bool act = i < M.end[blockIdx.x];
   double4 F;
-  force_mixed_body<K, ONE, false, false>(A, M, s, S, tab, i, lane, act, F);
+  force_mixed_body<K, ONE, false, false>(src_arena(A, S, st), A, M, s, S, tab, i, lane, act, F);
   double2 t = make_double2(1.e-16, 1.e-16);
-  BaAtom b;
-  b.on = false;
   if (act && lane == 0) {
-    A.force[i] = make_double4(F.x, F.y, F.z, 0.0);
-    A.epot[i] = F.w;
-    ba_calc(A, S, st, i, make_double4(F.x, F.y, F.z, 0.0), b);
-    t.x = b.d;
-    ba_store(A, S, st, i, b);
+    // (nobody sees the forces and energies of the steps inside a chunk)
+    ba_step(A, S, st, i, make_double4(F.x, F.y, F.z, 0.0), t);
   }
   skin_close<COND, false>(A, M, s, S, st, false, t, cond);
 }
@@ -3109,18 +3430,49 @@ __global__ void __launch_bounds__(BLOCK) k_smatb_force_fp64_ba(Arena A, BlockMap
   const int lane = threadIdx.x % K;
   const bool act = i < M.end[blockIdx.x];
   double4 F;
-  force_fp64_body<K, false, false>(A, M, s, S, tab, i, lane, act, F);
+  force_fp64_body<K, false, false>(src_arena(A, S, st), A, M, s, S, tab, i, lane, act, F);
   double2 t = make_double2(1.e-16, 1.e-16);
-  BaAtom b;
-  b.on = false;
   if (act && lane == 0) {
-    A.force[i] = make_double4(F.x, F.y, F.z, 0.0);
-    A.epot[i] = F.w;
-    ba_calc(A, S, st, i, make_double4(F.x, F.y, F.z, 0.0), b);
-    t.x = b.d;
-    ba_store(A, S, st, i, b);
+    // (nobody sees the forces and energies of the steps inside a chunk)
+    ba_step(A, S, st, i, make_double4(F.x, F.y, F.z, 0.0), t);
   }
   skin_close<COND, false>(A, M, s, S, st, false, t, cond);
+}
+
+// FIRE's per-atom mixing v = (1-a) v + a |v| F/|F| (FIRE.f90:99-114, with
+// |v|), after the atom's terms of P = sum v.F and of max |F|^2
+__device__ __forceinline__ void fire_mix(double al, const double4& F, double4& v, double& P, double& f2) {
+  P = v.x * F.x + v.y * F.y + v.z * F.z;
+  const double fn2 = F.x * F.x + F.y * F.y + F.z * F.z;
+  f2 = fn2;
+  const double vn = sqrt(v.x * v.x + v.y * v.y + v.z * v.z);
+  const double fn = sqrt(fn2);
+  const double mixf = fn > 0.0 ? al * vn / fn : 0.0;
+  v.x = v.x * (1.0 - al) + mixf * F.x;
+  v.y = v.y * (1.0 - al) + mixf * F.y;
+  v.z = v.z * (1.0 - al) + mixf * F.z;
+}
+
+// FIRE's dt / alpha control (FIRE.f90:116-131) from the system's P and max |F|^2
+__device__ __forceinline__ void fire_control(const SysDev& S, SysState& st, double Pt, double Ft) {
+  st.fire_P = Pt;
+  st.fmax2 = Ft;
+  st.fire_iter++;
+  const double alpha0 = 0.1, finc = 1.1, fdec = 0.5, falf = 0.99;
+  if (Pt > 0.0) {
+    st.fire_np++;
+    if (st.fire_np > 5) {
+      st.fire_dt = fmin(st.fire_dt * finc, S.fire_dtmax);
+      st.fire_alpha = st.fire_alpha * falf;
+    }
+  } else {
+    st.fire_np = 0;
+    st.fire_dt = st.fire_dt * fdec;
+    st.fire_alpha = alpha0;
+    st.fire_zero = 1;  // velocities are zeroed by the next step_a
+  }
+  const double fm = sqrt(Ft) * c_ui_ev();
+  if (fm < S.fire_fmax || st.fire_iter >= S.fire_maxit) st.fire_done = 1;
 }
 
 // integration_stepb (src/Integration.F90:264-301): velocity_verlet_b
@@ -3131,7 +3483,8 @@ __global__ void __launch_bounds__(BLOCK) k_smatb_force_fp64_ba(Arena A, BlockMap
 // MOVES: the launch includes systems whose step b moves the atoms (the
 // predictor-corrector, whose corrector also holds three more derivative
 // vectors, and Brownian dynamics); the other integrators' copy stays leaner
-template <bool MOVES>
+// W: the last half step of a chunk of fused steps (Ermak atoms come with w)
+template <bool MOVES, bool W = false>
 __global__ void __launch_bounds__(BLOCK) k_step_b(Arena A, BlockMap M) {
   int s = blk_sys(M);
   if (s < 0) return;  // padding block of a fixed-capacity map
@@ -3149,19 +3502,17 @@ __global__ void __launch_bounds__(BLOCK) k_step_b(Arena A, BlockMap M) {
     if (S.integ == IT_VV || S.integ == IT_FIRE) {
       vv_b_atom(S.integ == IT_FIRE ? st.fire_dt : S.dt, om, F, v, a);
       if (S.integ == IT_FIRE) {
-        P = v.x * F.x + v.y * F.y + v.z * F.z;
-        double fn2 = F.x * F.x + F.y * F.y + F.z * F.z;
-        f2max = fn2;
-        double vn = sqrt(v.x * v.x + v.y * v.y + v.z * v.z);
-        double fn = sqrt(fn2);
-        double al = st.fire_alpha;
-        double mixf = fn > 0.0 ? al * vn / fn : 0.0;
-        v.x = v.x * (1.0 - al) + mixf * F.x;
-        v.y = v.y * (1.0 - al) + mixf * F.y;
-        v.z = v.z * (1.0 - al) + mixf * F.z;
+        fire_mix(st.fire_alpha, F, v, P, f2max);
       }
     } else if (S.integ == IT_ERMAK) {
-      ermak_b_atom(S, om, F, A.vel_v[i], v, a);
+      if (W) {
+        v.x = ermak_v(S, om, F.x, v.x);
+        v.y = ermak_v(S, om, F.y, v.y);
+        v.z = ermak_v(S, om, F.z, v.z);
+        a.x = F.x * om; a.y = F.y * om; a.z = F.z * om;
+      } else {
+        ermak_b_atom(S, om, F, A.vel_v[i], v, a);
+      }
     } else if (S.integ == IT_LGF) {
       lgf_b_atom(S, om, F, A.vel_v[i], v, a);
     } else if (S.integ == IT_AXES) {
@@ -3212,7 +3563,7 @@ __global__ void __launch_bounds__(BLOCK) k_step_b(Arena A, BlockMap M) {
         v.z = (x.z - xo.z) / S.dt;
       }
       wrap_atom(S, x);
-      moved_atom(A, S, st, i, x, A.pos_old[i], A.type[i]);
+      moved_atom(A, S, st, i, x, A.pos_old[i], A.type[i], A.fxp);
     }
     A.vel[i] = v;
     A.acel[i] = a;
@@ -3247,26 +3598,7 @@ __global__ void __launch_bounds__(BLOCK) k_step_b(Arena A, BlockMap M) {
       Pt += __shfl_xor_sync(0xffffffffu, Pt, o);
       Ft = fmax(Ft, __shfl_xor_sync(0xffffffffu, Ft, o));
     }
-    if (threadIdx.x == 0 && !frozen) {
-      st.fire_P = Pt;
-      st.fmax2 = Ft;
-      st.fire_iter++;
-      const double alpha0 = 0.1, finc = 1.1, fdec = 0.5, falf = 0.99;
-      if (Pt > 0.0) {
-        st.fire_np++;
-        if (st.fire_np > 5) {
-          st.fire_dt = fmin(st.fire_dt * finc, S.fire_dtmax);
-          st.fire_alpha = st.fire_alpha * falf;
-        }
-      } else {
-        st.fire_np = 0;
-        st.fire_dt = st.fire_dt * fdec;
-        st.fire_alpha = alpha0;
-        st.fire_zero = 1;  // velocities are zeroed by the next step_a
-      }
-      double fm = sqrt(Ft) * c_ui_ev();
-      if (fm < S.fire_fmax || st.fire_iter >= S.fire_maxit) st.fire_done = 1;
-    }
+    if (threadIdx.x == 0 && !frozen) fire_control(S, st, Pt, Ft);
   }
 }
 

@@ -149,7 +149,7 @@ __global__ void k_neb_vv(Arena A, NebDev N, double dt) {
     const SysDev& S = A.sys[s];
     if (S.prec == PREC_MIXED || S.ff == FF_TERSOFF) {
       int bad = 0;
-      write_fx(A, S, i, x, A.type[i], bad);
+      write_fx(A.fxp, S, i, x, A.type[i], bad);
       if (bad) atomicOr(&A.st[s].status, ST_LOST);
     }
     if (!(x.x == x.x && x.y == x.y && x.z == x.z)) atomicOr(&A.st[s].status, ST_NAN);
