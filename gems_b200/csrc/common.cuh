@@ -240,6 +240,7 @@ struct Arena {
   int* chunk_sum;       // per 256-cell chunk
   int* cell_atoms;      // atom ids sorted by cell (descending within a cell)
   double4* cell_pos;    // their positions, in the same order (written with it at a rebuild)
+  float4* cell_rec;     // and in single precision, with the atom's id
   // Tersoff: rslot[m * cap + i] = the slot of i in the flist of its m-th
   // neighbour (255: none), built with the list; per step, tsmask[i] marks
   // the flist slots of i that are bonds and tsfb[a * cap + i] holds the force
@@ -254,6 +255,7 @@ struct Arena {
   double2* blk_top2;    // per-block top-2 displacement^2
   double* blk_red;      // per-block partial sums
   SysDev* sys;
+  SysDev* sys_b;        // the systems' records at their last list build
   SysState* st;
   PairP* prm;
   int* any_rebuild;     // OR over the systems of the last step

@@ -49,6 +49,7 @@ struct SysHost {
   bool first = true;        // next interact builds the list (update)
   bool pos_dirty = false;   // positions replaced from the host since the skin test
   bool has_forces = false;
+  bool built = false;       // the device holds a list (and the record of its build)
   int lanes = 8;            // lanes per atom in the force kernels (autotuned)
   int variant = 1;          // 1: species table in shared memory, 0: constants in
                             //    registers (single-species mixed SMA-TB; autotuned)
@@ -189,7 +190,7 @@ struct gemsgpu_pool {
   int64_t max_atoms = 0, max_cells = 0;
   int ff = 0, prec = 0, lanes = 8, variant = 1, chunk = 50;
   std::vector<int> active;  // system ids
-  // map kinds: 0 atoms/256, 1 cells/256, 2 atoms/LIST_ATOMS, 3 cells/8, 4 atoms/(256/K)
+  // map kinds: 0 atoms/256, 1 cells/256, 2 atoms/ROWS_ATOMS, 3 cells/8, 4 atoms/(256/K)
   int cap[5] = {0, 0, 0, 0, 0};
   int* dmap[5] = {nullptr, nullptr, nullptr, nullptr, nullptr};
   int* dsys = nullptr;      // padded system array
@@ -335,6 +336,7 @@ int grow_atoms(gemsgpu_ctx* ctx, int64_t need) {
   CHK(dgrow(ctx, &A.slot, keep, nc));
   CHK(dgrow(ctx, &A.cell_atoms, keep, nc));
   CHK(dgrow(ctx, &A.cell_pos, keep, nc));
+  CHK(dgrow(ctx, &A.cell_rec, keep, nc));
   CHK(dgrow(ctx, &A.ext_normals, 6 * keep, 6 * nc));
   // the lists' leading dimension is the atom capacity: re-lay them out
   if (A.lcap > 0) {
@@ -400,16 +402,21 @@ int list_smem_attr(gemsgpu_ctx* ctx, int lcap) {
   const size_t smem = list_smem(lcap), smemw = listw_smem<128>(lcap), smemw4 = listw_smem<512>(lcap);
   if (smem > 200 * 1024 || smemw > 200 * 1024 || smemw4 > 200 * 1024)
     return fail(ctx, GEMSGPU_ERR_ARG, "neighbour capacity %d too large", lcap);
+  if (lcap <= 384)
+    for (const void* fn : {(const void*)k_list_rows<1>, (const void*)k_list_rows<3>, (const void*)k_list_rows<9>})
+      CU(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                              (int)(ROWS_WARPS * rows_warp_bytes(lcap))));
   if (smem > 48 * 1024)
-    CU(cudaFuncSetAttribute(k_list_cells, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  if (smemw > 48 * 1024) {
-    CU(cudaFuncSetAttribute(k_list_cells_w<128, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smemw));
-    CU(cudaFuncSetAttribute(k_list_cells_w<128, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smemw));
-  }
-  if (smemw4 > 48 * 1024) {
-    CU(cudaFuncSetAttribute(k_list_cells_w<512, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smemw4));
-    CU(cudaFuncSetAttribute(k_list_cells_w<512, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smemw4));
-  }
+    for (const void* fn : {(const void*)k_list_cells<false>, (const void*)k_list_cells<true>})
+      CU(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  if (smemw > 48 * 1024)
+    for (const void* fn : {(const void*)k_list_cells_w<128, true, false>, (const void*)k_list_cells_w<128, false, false>,
+                           (const void*)k_list_cells_w<128, true, true>, (const void*)k_list_cells_w<128, false, true>})
+      CU(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smemw));
+  if (smemw4 > 48 * 1024)
+    for (const void* fn : {(const void*)k_list_cells_w<512, true, false>, (const void*)k_list_cells_w<512, false, false>,
+                           (const void*)k_list_cells_w<512, true, true>, (const void*)k_list_cells_w<512, false, true>})
+      CU(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smemw4));
   return 0;
 }
 
@@ -472,6 +479,7 @@ int grow_systems(gemsgpu_ctx* ctx, int need) {
   int nc = std::max(need, std::max(16, ctx->scap * 2));
   Arena& A = ctx->A;
   CHK(dgrow(ctx, &A.sys, ctx->scap, nc));
+  CHK(dgrow(ctx, &A.sys_b, ctx->scap, nc));
   CHK(dgrow(ctx, &A.st, ctx->scap, nc));
   CU(cudaMemsetAsync(A.st + ctx->scap, 0, (nc - ctx->scap) * sizeof(SysState), ctx->stream));
   if (ctx->h_st) cudaFreeHost(ctx->h_st);
@@ -950,26 +958,70 @@ int rebuild_grid(const gemsgpu_ctx* ctx, int nblk) { return std::max(1, std::min
 
 // the warp-per-cell list kernels for the systems of each tile size
 // (t128 / t512) and frame ([0] integer, [1] image)
-int launch_list_w(gemsgpu_ctx* ctx, const BlockMap& mc8, const bool* t128, const bool* t512) {
+template <bool REF>
+int launch_list_w(gemsgpu_ctx* ctx, const Arena& A, const BlockMap& mc8, const bool* t128, const bool* t512) {
   cudaStream_t st = ctx->stream;
-  const Arena& A = ctx->A;
   const int g = rebuild_grid(ctx, mc8.nblk);
-  if (t128[1]) k_list_cells_w<128, true><<<g, BLOCK, listw_smem<128>(A.lcap), st>>>(A, mc8);
-  if (t128[0]) k_list_cells_w<128, false><<<g, BLOCK, listw_smem<128>(A.lcap), st>>>(A, mc8);
-  if (t512[1]) k_list_cells_w<512, true><<<g, BLOCK, listw_smem<512>(A.lcap), st>>>(A, mc8);
-  if (t512[0]) k_list_cells_w<512, false><<<g, BLOCK, listw_smem<512>(A.lcap), st>>>(A, mc8);
+  if (t128[1]) k_list_cells_w<128, true, REF><<<g, BLOCK, listw_smem<128>(A.lcap), st>>>(A, mc8);
+  if (t128[0]) k_list_cells_w<128, false, REF><<<g, BLOCK, listw_smem<128>(A.lcap), st>>>(A, mc8);
+  if (t512[1]) k_list_cells_w<512, true, REF><<<g, BLOCK, listw_smem<512>(A.lcap), st>>>(A, mc8);
+  if (t512[0]) k_list_cells_w<512, false, REF><<<g, BLOCK, listw_smem<512>(A.lcap), st>>>(A, mc8);
   ctx->launches += t128[0] + t128[1] + t512[0] + t512[1];
   CU(cudaGetLastError());
   return 0;
 }
 
+void list_rows(gemsgpu_ctx* ctx, const BlockMap& m, int sp) {
+  const size_t sm = ROWS_WARPS * rows_warp_bytes(ctx->A.lcap);
+  const int nt = 32 * ROWS_WARPS;
+  const int g = (int)std::min<int64_t>((int64_t)m.nblk * rows_rounds(sp), 4 * ctx->nsm);
+  if (sp == 1) k_list_rows<1><<<g, nt, sm, ctx->stream>>>(ctx->A, m);
+  else if (sp == 3) k_list_rows<3><<<g, nt, sm, ctx->stream>>>(ctx->A, m);
+  else k_list_rows<9><<<g, nt, sm, ctx->stream>>>(ctx->A, m);
+  ++ctx->launches;
+}
+
+// the force lists of the systems that k_list_rows serves; a batch's systems
+// are rebuilt one or two at a time, so lanes per atom go by the largest
+int launch_list_rows(gemsgpu_ctx* ctx, const std::vector<int>& ss) {
+  int most = 0;
+  for (int s : ss)
+    if (rows_fit(ctx->sys[s].d, ctx->A.lcap)) most = std::max(most, ctx->sys[s].n);
+  if (!most || ctx->A.lcap > 384) return 0;
+  BlockMap m;
+  CHK(get_map(ctx, ss, ROWS_ATOMS, 0, &m));
+  list_rows(ctx, m, rows_split(most, 2 * ctx->nsm));
+  CU(cudaGetLastError());
+  return 0;
+}
+
+// the reference-order list kernels: for the systems that k_list_rows does not
+// serve, or with REF the reference's list alone for all of ss
+template <bool REF>
+int launch_ref_lists(gemsgpu_ctx* ctx, const std::vector<int>& ss, const Arena& A) {
+  BlockMap mc8, mc1;
+  CHK(get_map(ctx, ss, BLOCK / 32, 1, &mc8));
+  CHK(get_map(ctx, ss, 1, 1, &mc1));
+  bool kind[3][2] = {};
+  for (int s : ss) {
+    const SysDev& d = ctx->sys[s].d;
+    if (REF)  // (the build's record decides, on the device)
+      for (auto& k : kind) k[0] = k[1] = true;
+    else if (d.use_cells && !rows_fit(d, A.lcap)) kind[d.list_warp][d.list_img] = true;
+  }
+  if (kind[0][0] || kind[0][1]) {
+    k_list_cells<REF><<<rebuild_grid(ctx, mc1.nblk * LIST_SPLIT), BLOCK, list_smem(A.lcap), ctx->stream>>>(A, mc1);
+    ++ctx->launches;
+  }
+  return launch_list_w<REF>(ctx, A, mc8, kind[1], kind[2]);
+}
+
 int launch_rebuild(gemsgpu_ctx* ctx, const std::vector<int>& ss, int in_graph = 0) {
-  BlockMap ma, mc, mc8, mc1;
+  BlockMap ma, mc, mc8;
   const int* sa;
   CHK(get_map(ctx, ss, BLOCK, 0, &ma));
   CHK(get_map(ctx, ss, 256, 1, &mc));
   CHK(get_map(ctx, ss, BLOCK / 32, 1, &mc8));
-  CHK(get_map(ctx, ss, 1, 1, &mc1));
   CHK(sys_array(ctx, ss, &sa));
   cudaStream_t st = ctx->stream;
   const Arena& A = ctx->A;
@@ -982,14 +1034,8 @@ int launch_rebuild(gemsgpu_ctx* ctx, const std::vector<int>& ss, int in_graph = 
     k_scan2<<<(int)ss.size(), BLOCK, 0, st>>>(A, sa, (int)ss.size()); ++ctx->launches;
     k_scatter<<<ma.nblk, BLOCK, 0, st>>>(A, ma); ++ctx->launches;
     k_sort_cells<<<rebuild_grid(ctx, mc8.nblk), BLOCK, 0, st>>>(A, mc8); ++ctx->launches;
-    bool kind[3][2] = {};
-    for (int s : ss)
-      if (ctx->sys[s].d.use_cells) kind[ctx->sys[s].d.list_warp][ctx->sys[s].d.list_img] = true;
-    if (kind[0][0] || kind[0][1]) {
-      k_list_cells<<<rebuild_grid(ctx, mc1.nblk * LIST_SPLIT), BLOCK, list_smem(A.lcap), st>>>(A, mc1);
-      ++ctx->launches;
-    }
-    CHK(launch_list_w(ctx, mc8, kind[1], kind[2]));
+    CHK(launch_list_rows(ctx, ss));
+    CHK(launch_ref_lists<false>(ctx, ss, A));
   }
   if (n2) {
     k_list_n2<<<rebuild_grid(ctx, ma.nblk), BLOCK, 0, st>>>(A, ma); ++ctx->launches;
@@ -1222,31 +1268,15 @@ int estimate_cap(const SysHost& h) {
 }
 
 // ------------------------------------------------------------- teams
-template <int KIND, int MINB, bool RES>
-const void* team_fn_k(int K) {
-  switch (K) {
-    case 1: return (const void*)k_team<KIND, 1, MINB, RES>;
-    case 2: return (const void*)k_team<KIND, 2, MINB, RES>;
-    case 4: return (const void*)k_team<KIND, 4, MINB, RES>;
-    case 8: return (const void*)k_team<KIND, 8, MINB, RES>;
-    case 16: return (const void*)k_team<KIND, 16, MINB, RES>;
-    default: return (const void*)k_team<KIND, 32, MINB, RES>;
-  }
-}
-
-template <bool RES>
-const void* team_fn(int kind, int K) {
+const void* team_fn(int kind, int K, bool res) {
   switch (kind) {
-    case TK_LJ64: return team_fn_k<TK_LJ64, 2, RES>(K);
-    case TK_LJ32: return team_fn_k<TK_LJ32, 3, RES>(K);
-    case TK_SM64: return team_fn_k<TK_SM64, 2, RES>(K);
-    case TK_SM32: return team_fn_k<TK_SM32, 3, RES>(K);
-    default: return team_fn_k<TK_SM32R, 3, RES>(K);
+    case TK_LJ64: return team_fn_0(K, res);
+    case TK_LJ32: return team_fn_1(K, res);
+    case TK_SM64: return team_fn_2(K, res);
+    case TK_SM32: return team_fn_3(K, res);
+    case TK_SM32R: return team_fn_4(K, res);
+    default: return team_fn_ts(kind == TK_TS32, K);
   }
-}
-const void* team_fn_tersoff(bool mixed, int K) {
-  if (!mixed) return (const void*)k_team<TK_TS64, 4, 2, false>;
-  return K == 2 ? (const void*)k_team<TK_TS32, 2, 3, false> : (const void*)k_team<TK_TS32, 4, 3, false>;
 }
 
 constexpr int TEAM_MAX_CELLS = 12288;  // a CTA scans the system's cell counts in shared memory
@@ -1322,7 +1352,7 @@ int team_plan(gemsgpu_ctx* ctx, const std::vector<int>& ss) {
   const int apb = BLOCK / K;
   const bool one = h0.ntypes == 1;
   int maxcell = 0, big = 0;
-  bool w[2] = {false, false};
+  bool w[2] = {false, false};  // list builds: CTA per cell, rows
   int64_t total = 0, atoms = 0;
   for (int s : ss) {
     const SysHost& h = ctx->sys[s];
@@ -1333,7 +1363,7 @@ int team_plan(gemsgpu_ctx* ctx, const std::vector<int>& ss) {
     if (h.d.thermo != TH_NONE || h.d.virial || h.n == 0 || (h.ntypes == 1) != one) return 0;
     if (h.d.ncell > TEAM_MAX_CELLS) return 0;
     maxcell = std::max(maxcell, h.d.ncell);
-    if (h.d.use_cells) w[h.d.list_warp == 1] = true;
+    if (h.d.use_cells) w[rows_fit(h.d, ctx->A.lcap)] = true;
     big = std::max(big, h.n);
     total += (h.n + apb - 1) / apb;
   }
@@ -1345,8 +1375,9 @@ int team_plan(gemsgpu_ctx* ctx, const std::vector<int>& ss) {
   const bool ts = h0.d.ff == FF_TERSOFF;
   const size_t tsf = kind == TK_TS64 ? tsf_smem<double, 4>()
                      : kind == TK_TS32 ? (K == 2 ? tsf_smem<float, 2>() : tsf_smem<float, 4>()) : 0;
-  const size_t scratch = std::max(w[0] || !w[1] ? team_smem(ctx->A.lcap, maxcell, false, tsf) : (size_t)0,
-                                  w[1] ? team_smem(ctx->A.lcap, maxcell, true, tsf) : (size_t)0);
+  size_t scratch = 0;
+  for (int k = 0; k < 2; k++)
+    if (w[k]) scratch = std::max(scratch, team_smem(ctx->A.lcap, maxcell, k == 1, tsf));
   P.runs.clear();
   std::vector<int> all;  // per launch: its teams, then the team of each CTA
   std::vector<size_t> at_team, at_cta;
@@ -1376,7 +1407,7 @@ int team_plan(gemsgpu_ctx* ctx, const std::vector<int>& ss) {
   // 20 to 6.
   const int nmax = h0.d.ff == FF_LJ ? 16000 : 32000;
   int occ = 0;
-  const void* arena = ts ? team_fn_tersoff(mixed, K) : team_fn<false>(kind, K);
+  const void* arena = team_fn(kind, K, false);
   const size_t arena_sm = std::max(scratch, tsf);
   bool arena_ok = arena_sm <= (size_t)TEAM_SMEM && big <= nmax && (atoms <= nmax || big <= 5000);
   if (arena_ok) {
@@ -1385,7 +1416,7 @@ int team_plan(gemsgpu_ctx* ctx, const std::vector<int>& ss) {
     arena_ok = total <= (int64_t)occ * ctx->nsm;
   }
   std::vector<int> C;
-  const void* fn = ts || big > (arena_ok ? 640 : 2048) ? nullptr : team_fn<true>(kind, K);
+  const void* fn = ts || big > (arena_ok ? 640 : 2048) ? nullptr : team_fn(kind, K, true);
   if (fn && team_clusters(ctx, ss, fn, kind, apb, scratch, C)) {
     P.fn = fn;
     std::vector<size_t> order(ss.size());  // the largest first
@@ -1571,6 +1602,7 @@ int interact_group(gemsgpu_ctx* ctx, const std::vector<int>& ss, bool sync_check
   for (int s : ss) {
     SysHost& h = ctx->sys[s];
     h.first = false;
+    h.built = true;
     h.pos_dirty = false;
     h.has_forces = true;
   }
@@ -1841,6 +1873,7 @@ int get_graph(gemsgpu_ctx* ctx, const std::vector<int>& ss, int nsteps, cudaGrap
     CHK(get_map(ctx, ss, 256, 1, &m));
     CHK(get_map(ctx, ss, BLOCK / 32, 1, &m));
     CHK(get_map(ctx, ss, 1, 1, &m));
+    CHK(get_map(ctx, ss, ROWS_ATOMS, 0, &m));
     CHK(sys_array(ctx, ss, &sa));
     const size_t nbr = std::min(ss.size(), MAX_BRANCHES);
     for (size_t j = 0; j < nbr && ss.size() > 1; j++)
@@ -1950,6 +1983,7 @@ void settled(gemsgpu_ctx* ctx, const std::vector<int>& ss) {
   for (int s : ss) {
     SysHost& h = ctx->sys[s];
     h.first = false;
+    h.built = true;
     h.pos_dirty = false;
     h.has_forces = true;
   }
@@ -2080,7 +2114,7 @@ int pool_kind_apb(const gemsgpu_pool* P, int kind) {
   switch (kind) {
     case 0: return BLOCK;
     case 1: return 256;
-    case 2: return LIST_ATOMS;
+    case 2: return ROWS_ATOMS;
     case 3: return BLOCK / 32;
     default: return BLOCK / P->lanes;
   }
@@ -2177,10 +2211,11 @@ int pool_rebuild(gemsgpu_pool* P, int in_graph) {
   k_scan2<<<ns, BLOCK, 0, st>>>(A, P->dsys, ns); ++ctx->launches;
   k_scatter<<<ma.nblk, BLOCK, 0, st>>>(A, ma); ++ctx->launches;
   k_sort_cells<<<rebuild_grid(ctx, mc8.nblk), BLOCK, 0, st>>>(A, mc8); ++ctx->launches;
-  k_list_cells<<<rebuild_grid(ctx, mc8.nblk * LIST_SPLIT), BLOCK, list_smem(A.lcap), st>>>(A, mc8);
+  k_list_cells<false><<<rebuild_grid(ctx, mc8.nblk * LIST_SPLIT), BLOCK, list_smem(A.lcap), st>>>(A, mc8);
   ++ctx->launches;
   const bool all[2] = {true, true};
-  CHK(launch_list_w(ctx, mc8, all, all));
+  CHK(launch_list_w<false>(ctx, A, mc8, all, all));
+  if (A.lcap <= 384) list_rows(ctx, P->maps[2], 1);
   k_list_n2<<<rebuild_grid(ctx, ma.nblk), BLOCK, 0, st>>>(A, ma); ++ctx->launches;
   if (P->ff == FF_TERSOFF) {
     k_tsf_rslot<<<rebuild_grid(ctx, ma.nblk), BLOCK, 0, st>>>(A, ma); ++ctx->launches;
@@ -2425,7 +2460,7 @@ int gemsgpu_destroy(gemsgpu_ctx* ctx) {
   void* ptrs[] = {A.pos, A.pos_old, A.vel, A.acel, A.force, A.vel_v, A.acel2, A.acel3, A.acel4, A.epot, A.band, A.eband,
                   A.ebandf, A.fxp, A.pose, A.pose2, A.fxe, A.minv, A.mass, A.type, A.nn, A.hnn, A.ncut, A.list, A.flist, A.cell_of, A.slot,
                   A.cell_count, A.cell_n, A.cell_loc, A.cell_start, A.chunk_sum, A.cell_atoms,
-                  A.cell_pos, A.rslot, A.tidx, A.tsmask, A.tsfb, A.tsfb32,
+                  A.cell_pos, A.cell_rec, A.sys_b, A.rslot, A.tidx, A.tsmask, A.tsfb, A.tsfb32,
                   A.ext_normals, A.blk_top2, A.blk_red, A.sys, A.st, A.prm, A.any_rebuild, A.body_runs,
                   ctx->d_red, ctx->snap, ctx->snap_st, ctx->snap_sys, ctx->d_sys,
                   ctx->lbw.x0, ctx->lbw.g, ctx->lbw.gold, ctx->lbw.d, ctx->lbw.S, ctx->lbw.Y, ctx->lbw.st,
@@ -2553,6 +2588,7 @@ int gemsgpu_upload(gemsgpu_ctx* ctx, int sys, const double* pos, const double* v
   CHK(get_map(ctx, {sys}, BLOCK, 0, &m));
   k_refresh_fx<<<m.nblk, BLOCK, 0, ctx->stream>>>(A, m); ++ctx->launches;
   h.first = true;
+  h.built = false;
   h.has_forces = false;
   CU(cudaGetLastError());
   return 0;
@@ -2824,13 +2860,33 @@ int gemsgpu_update(gemsgpu_ctx* ctx, int sys) {
   }
   CHK(status_error(ctx, sys, ctx->h_st[sys].status));
   ctx->sys[sys].first = false;
+  ctx->sys[sys].built = true;
   ctx->sys[sys].pos_dirty = false;
+  return 0;
+}
+
+// Write the reference's list of system sys at its last build: the
+// reference-order kernels on that build's cells, positions (pos_old) and box.
+static int reference_list(gemsgpu_ctx* ctx, int sys) {
+  const std::vector<int> ss{sys};
+  CHK(read_states(ctx));
+  const int flag = ctx->h_st[sys].rebuild;
+  Arena B = ctx->A;
+  B.sys = ctx->A.sys_b;
+  B.pos = ctx->A.pos_old;
+  const int* sa;
+  CHK(sys_array(ctx, ss, &sa));
+  k_force_rebuild<<<1, 256, 0, ctx->stream>>>(ctx->A, sa, 1); ++ctx->launches;
+  CHK(launch_ref_lists<true>(ctx, ss, B));
+  CU(cudaMemcpyAsync(&ctx->A.st[sys].rebuild, &flag, sizeof(int), cudaMemcpyHostToDevice, ctx->stream));
+  CU(cudaStreamSynchronize(ctx->stream));
   return 0;
 }
 
 int gemsgpu_get_list(gemsgpu_ctx* ctx, int sys, int* nn, int* list, int cap, int* cap_needed) {
   CHK(check_sys(ctx, sys));
   const SysHost& h = ctx->sys[sys];
+  if (h.built && h.d.use_cells) CHK(reference_list(ctx, sys));
   std::vector<int> hn(h.n);
   // a half-list system's `list` holds the half list (hnn entries); flist
   // holds the full list the force kernels use

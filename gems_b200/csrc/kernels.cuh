@@ -365,7 +365,7 @@ __device__ __forceinline__ void skin_finish(const Arena& A, const BlockMap& M, i
   }
 }
 
-__global__ void k_skin(Arena A, BlockMap M) {
+static __global__ void k_skin(Arena A, BlockMap M) {
   int s = blk_sys(M);
   if (s < 0) return;  // padding block of a fixed-capacity map
   int i = M.first[blockIdx.x] + threadIdx.x;
@@ -376,7 +376,7 @@ __global__ void k_skin(Arena A, BlockMap M) {
 }
 
 // mark systems for rebuild (first interact: update(), Interaction.f90:174)
-__global__ void k_force_rebuild(Arena A, const int* sys, int nsys) {
+static __global__ void k_force_rebuild(Arena A, const int* sys, int nsys) {
   int k = blockIdx.x * blockDim.x + threadIdx.x;
   if (k < nsys && sys[k] >= 0) {
     A.st[sys[k]].rebuild = 1;
@@ -385,7 +385,7 @@ __global__ void k_force_rebuild(Arena A, const int* sys, int nsys) {
 }
 
 // clear the per-chunk status words of a set of systems
-__global__ void k_clear_status(Arena A, const int* sys, int nsys) {
+static __global__ void k_clear_status(Arena A, const int* sys, int nsys) {
   int k = blockIdx.x * blockDim.x + threadIdx.x;
   if (k < nsys && sys[k] >= 0) {
     A.st[sys[k]].status = 0;
@@ -394,7 +394,7 @@ __global__ void k_clear_status(Arena A, const int* sys, int nsys) {
 }
 
 // refresh fixed-point positions (after an upload or set_positions)
-__global__ void k_refresh_fx(Arena A, BlockMap M) {
+static __global__ void k_refresh_fx(Arena A, BlockMap M) {
   int s = blk_sys(M);
   if (s < 0) return;  // padding block of a fixed-capacity map
   int i = M.first[blockIdx.x] + threadIdx.x;
@@ -423,7 +423,7 @@ __device__ __forceinline__ int atom_cell(const Arena& A, int s, const SysDev& S,
   return S.cell_off + c0 + S.nc[0] * (c1 + S.nc[1] * c2);
 }
 
-__global__ void k_bin(Arena A, BlockMap M) {
+static __global__ void k_bin(Arena A, BlockMap M) {
   int s = blk_sys(M);
   if (s < 0) return;  // padding block of a fixed-capacity map
   const SysDev& S = A.sys[s];
@@ -436,7 +436,7 @@ __global__ void k_bin(Arena A, BlockMap M) {
 }
 
 // per 256-cell chunk: local exclusive prefix, chunk total; resets counts
-__global__ void k_scan1(Arena A, BlockMap C) {
+static __global__ void k_scan1(Arena A, BlockMap C) {
   int s = blk_sys(C);
   if (s < 0) return;  // padding block of a fixed-capacity map
   if (!A.st[s].rebuild || !A.sys[s].use_cells) return;
@@ -461,7 +461,7 @@ __global__ void k_scan1(Arena A, BlockMap C) {
 }
 
 // one block per system: exclusive prefix of its chunk totals
-__global__ void k_scan2(Arena A, const int* sys, int nsys) {
+static __global__ void k_scan2(Arena A, const int* sys, int nsys) {
   int s = sys[blockIdx.x];
   if (s < 0) return;
   const SysDev& S = A.sys[s];
@@ -492,7 +492,7 @@ __global__ void k_scan2(Arena A, const int* sys, int nsys) {
   }
 }
 
-__global__ void k_scatter(Arena A, BlockMap M) {
+static __global__ void k_scatter(Arena A, BlockMap M) {
   int s = blk_sys(M);
   if (s < 0) return;  // padding block of a fixed-capacity map
   if (!A.st[s].rebuild || !A.sys[s].use_cells) return;
@@ -515,12 +515,13 @@ __global__ void k_scatter(Arena A, BlockMap M) {
 // batch, or of a system with many cells, thus costs its work plus one
 // parallel test per BLOCK items, not a launch or a serial test per item.
 // Items are independent, so the order in which a CTA takes them is free.
-template <class Check, class Body>
+// (NT: threads of a CTA)
+template <int NT = BLOCK, class Check, class Body>
 __device__ __forceinline__ void rebuild_items(int nitems, Check live, Body body) {
-  __shared__ int items[BLOCK];
+  __shared__ int items[NT];
   __shared__ int nlive;
   const int G = gridDim.x;
-  for (int base = 0; (int64_t)blockIdx.x + (int64_t)base * G < nitems; base += BLOCK) {
+  for (int base = 0; (int64_t)blockIdx.x + (int64_t)base * G < nitems; base += NT) {
     const int64_t w = (int64_t)blockIdx.x + (int64_t)(base + threadIdx.x) * G;
     if (threadIdx.x == 0) nlive = 0;
     __syncthreads();
@@ -536,6 +537,30 @@ __device__ __forceinline__ void rebuild_items(int nitems, Check live, Body body)
 __device__ __forceinline__ bool rebuild_block(const Arena& A, const BlockMap& M, int b, bool cells) {
   const int s = M.sys[b];
   return s >= 0 && A.st[s].rebuild && (A.sys[s].use_cells != 0) == cells;
+}
+// Systems whose force lists k_list_rows builds: three cells or more in every
+// dimension (a row's cells are distinct), few atoms a cell, and a box that stays.
+// Measured, one rebuild, warp or CTA per cell -> rows: 1M Si (3 a cell) 1.40 ->
+// 0.75 ms; but 8 x 32k Au (15 a cell) 0.61 -> 0.63 ms, 16 x 4000 LJ (32 a cell)
+// 0.31 -> 0.38.
+__host__ __device__ __forceinline__ bool rows_fit(const SysDev& S, int lcap) {
+  return S.use_cells && S.nc[0] >= 3 && S.nc[1] >= 3 && S.nc[2] >= 3 && lcap <= 384 && S.n < 6 * (int64_t)S.ncell &&
+         S.integ != IT_LGF && S.integ != IT_AXES && S.integ != IT_LKD;
+}
+
+// a block whose reference list is due: for REF every flagged system's, else
+// those whose force lists come with it
+template <bool REF>
+__device__ __forceinline__ bool ref_list_block(const Arena& A, const BlockMap& M, int b) {
+  return rebuild_block(A, M, b, true) && (REF || !rows_fit(A.sys[M.sys[b]], A.lcap));
+}
+
+// atom i at place p of the cell order: its position, and in single precision
+// (with the atom's id) for the list kernel's filter
+__device__ __forceinline__ void put_cell(const Arena& A, int p, int i) {
+  const double4 x = A.pos[i];
+  A.cell_pos[p] = x;
+  A.cell_rec[p] = make_float4((float)x.x, (float)x.y, (float)x.z, __int_as_float(i));
 }
 
 // one warp orders the n atoms of the cell whose atoms start at `start`
@@ -560,11 +585,11 @@ __device__ __forceinline__ void sort_cell(const Arena& A, int start, int n, int 
     // each lane places its own atoms (id and position) at their ranks
     if (ln < n) {
       a[r0] = v0;
-      A.cell_pos[start + r0] = A.pos[v0];
+      put_cell(A, start + r0, v0);
     }
     if (ln + 32 < n) {
       a[r1] = v1;
-      A.cell_pos[start + r1] = A.pos[v1];
+      put_cell(A, start + r1, v1);
     }
   } else if (ln == 0) {
     for (int x = 1; x < n; x++) {
@@ -576,11 +601,11 @@ __device__ __forceinline__ void sort_cell(const Arena& A, int start, int n, int 
       }
       a[y + 1] = v;
     }
-    for (int x = 0; x < n; x++) A.cell_pos[start + x] = A.pos[a[x]];  // the lane's own writes
+    for (int x = 0; x < n; x++) put_cell(A, start + x, a[x]);  // the lane's own writes
   }
 }
 
-__global__ void k_sort_cells(Arena A, BlockMap C) {
+static __global__ void k_sort_cells(Arena A, BlockMap C) {
   rebuild_items(C.nblk, [&](int b) { return rebuild_block(A, C, b, true); }, [&](int b) {
     const int warp = threadIdx.x >> 5, ln = threadIdx.x & 31;
     const int first = C.first[b], end = C.end[b];
@@ -706,6 +731,8 @@ __device__ __forceinline__ int live_entries(const Arena& A, int lk, int i, int n
 // order: ids, bit 31 set on the entries a half list leaves out, and r^2 as
 // float, within err of the exact r^2) out to the arena: `list` in the
 // reference's order, `flist` in the force order, the skip counts and nn / hnn.
+// REF: the reference's list alone (`list` and hnn).
+template <bool REF>
 __device__ __forceinline__ void list_row_out(const Arena& A, const SysDev& S, int s, int i, int m,
                                              const int* row, const float* rrow, float err, int* boff, int ln) {
   const int n = min(m, A.lcap);
@@ -718,8 +745,12 @@ __device__ __forceinline__ void list_row_out(const Arena& A, const SysDev& S, in
     if (h) A.list[(size_t)(mh + __popc(hb & ((1u << ln) - 1u))) * A.cap + i] = row[e];
     mh += __popc(hb);
   }
-  list_force_order(A, S, i, n, row, rrow, err, boff, ln);
-  if (ln == 0) list_done(A, s, i, m, mh, false);
+  if constexpr (REF) {
+    if (ln == 0) A.hnn[i] = mh;
+  } else {
+    list_force_order(A, S, i, n, row, rrow, err, boff, ln);
+    if (ln == 0) list_done(A, s, i, m, mh, false);
+  }
 }
 
 // ---- the candidate test of the cell-list builds
@@ -921,7 +952,7 @@ __host__ __device__ constexpr size_t list_smem(int lcap) {
 
 // (TILE: candidates staged at a time; the CTA takes the atom passes part,
 // part + nparts, ... of the cells [c0, c1) of system s)
-template <bool IMG, int TILE>
+template <bool IMG, int TILE, bool REF = false>
 __device__ __forceinline__ void list_cells_item(const Arena& A, int s, const SysDev& S, int c0, int c1, int part,
                                                 int nparts, float4* cf, int* stage, float* stage_rd, int* nb_start,
                                                 int* nb_pref, double3* nb_sh, int* boff) {
@@ -973,7 +1004,7 @@ __device__ __forceinline__ void list_cells_item(const Arena& A, int s, const Sys
         const int j = A.cell_atoms[idx];
         const double4 p = A.cell_pos[idx];
         cf[q] = list_record<IMG>(f, p, j, nb_sh[k], o);
-        if (g < own) A.pos_old[j] = p;  // the home cell's atoms: the list's reference positions
+        if (!REF && g < own) A.pos_old[j] = p;  // the home cell's atoms: the list's reference positions
       }
     };
     const bool one = T <= TILE;  // one tile stays staged for all this CTA's passes
@@ -1008,13 +1039,14 @@ __device__ __forceinline__ void list_cells_item(const Arena& A, int s, const Sys
         if (act) list_scan_tile<IMG>(A, S, f, cf, t0, tn, i, a, ri, half, own, hend, row, rrow, A.lcap, m, ln);
       }
       __syncwarp();
-      if (act) list_row_out(A, S, s, i, m, row, rrow, f.err, boff, ln);
+      if (act) list_row_out<REF>(A, S, s, i, m, row, rrow, f.err, boff, ln);
       __syncwarp();
     }
     __syncthreads();  // nb_* and the tile are rewritten for the next cell
   }
 }
 
+template <bool REF>
 __global__ void __launch_bounds__(BLOCK) k_list_cells(Arena A, BlockMap C) {
   extern __shared__ __align__(16) unsigned char list_sh[];
   float4* cf = reinterpret_cast<float4*>(list_sh);                          // LIST_TILE records
@@ -1031,7 +1063,7 @@ __global__ void __launch_bounds__(BLOCK) k_list_cells(Arena A, BlockMap C) {
   // over every CTA whatever the grid size
   auto live = [&](int w) {
     const int b = w % C.nblk, part = w / C.nblk;
-    if (!rebuild_block(A, C, b, true) || A.sys[C.sys[b]].list_warp) return false;
+    if (!ref_list_block<REF>(A, C, b) || A.sys[C.sys[b]].list_warp) return false;
     // one-cell blocks: is there an atom pass for this part?
     return C.end[b] - C.first[b] != 1 || part * LIST_ATOMS < A.cell_n[C.first[b]];
   };
@@ -1040,10 +1072,10 @@ __global__ void __launch_bounds__(BLOCK) k_list_cells(Arena A, BlockMap C) {
     const int s = C.sys[b], c0 = C.first[b], c1 = C.end[b];
     const SysDev& S = A.sys[s];
     if (S.list_img)
-      list_cells_item<true, LIST_TILE>(A, s, S, c0, c1, part, LIST_SPLIT, cf, stage, stage_rd, nb_start, nb_pref,
+      list_cells_item<true, LIST_TILE, REF>(A, s, S, c0, c1, part, LIST_SPLIT, cf, stage, stage_rd, nb_start, nb_pref,
                                        nb_sh, boff_sh[warp]);
     else
-      list_cells_item<false, LIST_TILE>(A, s, S, c0, c1, part, LIST_SPLIT, cf, stage, stage_rd, nb_start, nb_pref,
+      list_cells_item<false, LIST_TILE, REF>(A, s, S, c0, c1, part, LIST_SPLIT, cf, stage, stage_rd, nb_start, nb_pref,
                                         nb_sh, boff_sh[warp]);
   });
 }
@@ -1068,12 +1100,16 @@ __host__ __device__ constexpr size_t listw_smem(int lcap) {
   return (size_t)(BLOCK / 32) * listw_warp_bytes<TILE>(lcap);
 }
 
-template <bool IMG, int TILE>
-__device__ __forceinline__ void list_cells_w_item(const Arena& A, int s, const SysDev& S, int c, float4* cf, int* boff,
+template <bool IMG, int TILE, bool REF = false>
+__device__ __forceinline__ void list_cells_w_item(const Arena& A, const BlockMap& C, int b, float4* cf, int* boff,
                                                   int* row, float* rrow) {
   constexpr int U = 2;  // loads in flight per lane while staging
-  const int ln = threadIdx.x & 31;
+  const int warp = threadIdx.x >> 5, ln = threadIdx.x & 31;
   const unsigned FULL = 0xffffffffu;
+  const int c = C.first[b] + warp;
+  if (c >= C.end[b]) return;  // warp-uniform
+  const int s = C.sys[b];
+  const SysDev& S = A.sys[s];
   const ListFrame f = list_frame(S);
   const bool half = S.half != 0;
   const int cl = c - S.cell_off;
@@ -1136,7 +1172,7 @@ __device__ __forceinline__ void list_cells_w_item(const Arena& A, int s, const S
                              __shfl_sync(FULL, sh.z, kv[u]));
         if (q < tn) {
           cf[q] = list_record<IMG>(f, p[u], jv[u], shk, o);
-          if (t0 + q < own) A.pos_old[jv[u]] = p[u];  // the home cell's atoms: the list's reference positions
+          if (!REF && t0 + q < own) A.pos_old[jv[u]] = p[u];  // the home cell's atoms: the list's reference positions
         }
       }
     }
@@ -1159,7 +1195,7 @@ __device__ __forceinline__ void list_cells_w_item(const Arena& A, int s, const S
       list_scan_tile<IMG>(A, S, f, cf, t0, tn, i, a, ri, half, own, hend, row, rrow, A.lcap, m, ln);
     }
     __syncwarp();
-    list_row_out(A, S, s, i, m, row, rrow, f.err, boff, ln);
+    list_row_out<REF>(A, S, s, i, m, row, rrow, f.err, boff, ln);
     __syncwarp();
   }
 }
@@ -1167,7 +1203,7 @@ __device__ __forceinline__ void list_cells_w_item(const Arena& A, int s, const S
 // register bounds measured best: two blocks per SM for both tiles (three
 // blocks of the 128 tile spill the staging's positions; the 512 tile's
 // 72 KB of tiles fit three, but more registers win)
-template <int TILE, bool IMG>
+template <int TILE, bool IMG, bool REF>
 __global__ void __launch_bounds__(BLOCK, 2) k_list_cells_w(Arena A, BlockMap C) {
   extern __shared__ __align__(16) unsigned char listw_sh[];
   const int warp = threadIdx.x >> 5;
@@ -1178,19 +1214,272 @@ __global__ void __launch_bounds__(BLOCK, 2) k_list_cells_w(Arena A, BlockMap C) 
   float* rrow = reinterpret_cast<float*>(row + A.lcap);
   constexpr int KIND = TILE == 128 ? 1 : 2;  // SysDev::list_warp of the systems this kernel builds
   rebuild_items(C.nblk, [&](int b) {
-      if (!rebuild_block(A, C, b, true)) return false;
+      if (!ref_list_block<REF>(A, C, b)) return false;
       const SysDev& S = A.sys[C.sys[b]];
       return S.list_warp == KIND && (S.list_img != 0) == IMG;
-    }, [&](int b) {
-      const int c = C.first[b] + warp;
-      if (c < C.end[b]) list_cells_w_item<IMG, TILE>(A, C.sys[b], A.sys[C.sys[b]], c, cf, boff, row, rrow);  // warp-uniform
+    }, [&](int b) { list_cells_w_item<IMG, TILE, REF>(A, C, b, cf, boff, row, rrow); });
+}
+
+// ---- the force lists of a step, one thread an atom
+// The kernels above write the reference's list in the reference's order.  The
+// force kernels need only flist, in any fixed order within a band, so while
+// the atoms move this kernel writes flist alone (gemsgpu_get_list asks the
+// kernels above for the reference's list).  A warp takes 32 atoms that follow
+// one another in the cell order, so its lanes' cells are few and adjacent, and
+// each lane walks its own 27 cells: in the cell order the three cells of a row
+// along x are one run (two where the row wraps), so a lane has nine runs of
+// consecutive 16-byte records, and lanes of one cell read the same addresses.
+// No candidate is staged and no ballot or prefix is needed: a lane appends what
+// it accepts to its own column of shared memory (slot x lane: no bank
+// conflicts).  About 20 instructions per 32 candidates, where a warp per atom
+// took 30 plus 400 per atom to place the row by ballots (measured: see
+// k_list_rows).
+//
+// An accepted candidate is kept in 32 bits: the upper half of r^2 as float (a
+// monotone code, 0.8 % wide) and its place, as the run (5 bits) and the place in
+// the run (11 bits; a longer run sends the system to the kernels above, as a
+// list of more than 384 entries does).  The second phase counts the entries
+// per band and writes the row band by band.  An entry counts below a skip
+// threshold if its code is at most the threshold's, so in a code's width
+// above the threshold it still counts as below: the force kernels then visit
+// an entry more, never one less.
+//
+// The filter's coordinates are single-precision copies of the positions, each
+// component off by at most 2^-24 of L, the image shift is subtracted from the
+// atom's own FP64 coordinate before it is rounded, and the difference and sum
+// round as in ListFrame: |r2f - r^2| <= rows_err near rlist, inside which the
+// exact predicate decides.
+//
+// SP lanes share an atom (1, 3 or 9, fewer atoms needing more): each takes 9 / SP
+// of its rows, so small systems still have a thousand warps at work.  The row
+// lists a band's entries lane by lane, that is run by run whatever SP is.
+constexpr int ROWS_WARPS = 4;    // warps of a CTA of k_list_rows: adjacent atoms, whose runs overlap in L1
+constexpr int ROWS_ATOMS = 120;  // atoms of a block of its map: 30 / SP a warp, 1, 3 or 10 rounds
+__host__ __device__ constexpr int rows_per_warp(int sp) { return sp == 1 ? 30 : sp == 3 ? 10 : 3; }
+__host__ __device__ constexpr int rows_rounds(int sp) { return sp == 1 ? 1 : sp == 3 ? 3 : 10; }
+// lanes per atom for n atoms on `warps` warps
+__host__ __device__ constexpr int rows_split(int64_t n, int64_t warps) {
+  return n >= 30 * warps ? 1 : n >= 10 * warps ? 3 : 9;
+}
+constexpr int ROWS_RUN = 2048;  // places of a run that a code can name
+__host__ __device__ __forceinline__ int rows_split(int n) { return n > 37888 ? 1 : n > 18944 ? 2 : n > 9472 ? 4 : 8; }
+__host__ __device__ constexpr size_t rows_warp_bytes(int lcap) {
+  return (size_t)32 * (lcap + 10 + 18) * sizeof(int);  // entries, bands, run starts
+}
+struct RowsFrame {
+  float lo, hi;      // r2f < lo: inside rlist; r2f >= hi: outside
+  unsigned code[9];  // of the force order's split and the skip thresholds
+};
+__device__ __forceinline__ RowsFrame rows_frame(const SysDev& S) {
+  RowsFrame f;
+  double sd = 0.0, sd2 = 0.0, dm = 0.0;
+#pragma unroll
+  for (int k = 0; k < 3; k++) {
+    const double dk = 4.0 * 5.9604644775390625e-8 * (S.L[k] + S.rlist);
+    sd += dk;
+    sd2 += dk * dk;
+    dm = fmax(dm, dk);
+  }
+  const double err = 2.0 * (S.rlist + dm) * sd + sd2 + 1e-6 * S.rlist2;
+  f.lo = __double2float_rd(S.rlist2 - err);
+  f.hi = __double2float_ru(S.rlist2 + err);
+  f.code[0] = __float_as_uint(S.nsplit_r2) >> 16;
+#pragma unroll
+  for (int k = 0; k < 8; k++) f.code[k + 1] = __float_as_uint(__fadd_ru(S.ncut_r2[k], __double2float_ru(err))) >> 16;
+  f.code[0] = min(f.code[0], f.code[1]);
+  return f;
+}
+
+// The rows of the atoms at places p0, p0 + 1, ... (rows_per_warp(SP), to pend)
+// of system s's cell order, by one warp.  buf: rows_warp_bytes(A.lcap) of
+// shared memory.
+template <int SP>
+__device__ __forceinline__ void list_rows_warp(const Arena& A, int s, const SysDev& S, const RowsFrame& fr, int p0,
+                                               int pend, int* buf, int ln) {
+  constexpr int RPL = 9 / SP;  // rows of a lane
+  const unsigned FULL = 0xffffffffu;
+  const int lcap = A.lcap, own = ln / SP, part = ln % SP, p = p0 + own;
+  const bool act = own < rows_per_warp(SP) && p < pend;
+  int* col = buf + ln;                   // slot e at col[32 e]
+  int* hist = buf + 32 * lcap + ln;      // band b at hist[32 b]
+  int* start = hist + 32 * 10;           // run r at start[32 r]
+  const float flo = fr.lo, fhi = fr.hi;
+  int i = -1, m = 0, cx = 1, cy = 1, cz = 1;
+  double4 x = make_double4(0, 0, 0, 0);
+  if (act) {
+    i = A.cell_atoms[p];
+    x = A.cell_pos[p];
+    if (part == 0) A.pos_old[i] = x;
+    cell_xyz(S, A.cell_of[i] - S.cell_off, cx, cy, cz);
+  }
+  const int nx = S.nc[0], ny = S.nc[1], nz = S.nc[2];
+  const int x0 = max(cx - 1, 0), x1 = min(cx + 1, nx - 1);
+  const int wx = !act || !S.pbc[0] ? -1 : cx == 0 ? nx - 1 : cx == nx - 1 ? 0 : -1;  // the cell across the face
+  const float ax = (float)x.x, wax = (float)(x.x - (wx > 0 ? -S.L[0] : S.L[0]));
+  const int nw = __any_sync(FULL, wx >= 0) ? 2 : 1;
+  // run k = 2 row + w: the row's run (w = 0), then the wrapped cell's (w = 1)
+  auto bounds = [&](int rr, int w, int& b, int& e, float& ay, float& az) {
+    const int r = part * RPL + rr, dz = r / 3 - 1, dy = r - 3 * (dz + 1) - 1;
+    int y = cy + dy, z = cz + dz;
+    double sy = 0.0, sz = 0.0;
+    bool ok = act;
+    if (z < 0) z += nz, sz = -S.L[2], ok = ok && S.pbc[2];
+    else if (z >= nz) z -= nz, sz = S.L[2], ok = ok && S.pbc[2];
+    if (y < 0) y += ny, sy = -S.L[1], ok = ok && S.pbc[1];
+    else if (y >= ny) y -= ny, sy = S.L[1], ok = ok && S.pbc[1];
+    az = (float)(x.z - sz);
+    ay = (float)(x.y - sy);
+    const int row = S.cell_off + nx * (y + ny * z);
+    b = e = 0;
+    if (ok && (w == 0 || wx >= 0)) {
+      const int c0 = row + (w ? wx : x0), c1 = row + (w ? wx : x1);
+      b = A.cell_start[c0];
+      e = A.cell_start[c1] + A.cell_n[c1];
+    }
+  };
+  int nb, ne;
+  float nay, naz;
+  bounds(0, 0, nb, ne, nay, naz);
+#pragma unroll 1
+  for (int k = 0; k < RPL * nw; k++) {
+    const int rr = nw == 2 ? k >> 1 : k, w = nw == 2 ? k & 1 : 0;
+    const int b = nb, e = ne;
+    const float ay = nay, az = naz, bx = w ? wax : ax;
+    if (k + 1 < RPL * nw) bounds(nw == 2 ? (k + 1) >> 1 : k + 1, nw == 2 ? (k + 1) & 1 : 0, nb, ne, nay, naz);  // in flight meanwhile
+    start[32 * (2 * rr + w)] = b;
+    if (e - b > ROWS_RUN) m = max(m, 385);  // (with lcap <= 384: a list overflow)
+    const unsigned tag = (unsigned)(2 * rr + w) << 11;
+    auto dist = [&](const float4& c) {
+      const float u = c.x - bx, v = c.y - ay, t = c.z - az;
+      return fmaf(t, t, fmaf(v, v, u * u));
+    };
+    // the exact predicate, within the error bound of rlist
+    auto exact = [&](float r2, int q) {
+      const double rd = rd_exact(S, x, A.cell_pos[q]);
+      return rd < S.rlist2 ? (float)rd : fhi;
+    };
+    auto take = [&](float r2, int q) {
+      const bool in = r2 < fhi && q != p;
+      if (in && m < lcap) col[32 * m] = (int)((__float_as_uint(r2) & 0xffff0000u) | tag | ((unsigned)(q - b) & 2047u));
+      m += in;
+    };
+    // four candidates at a time, the next four's records in flight
+    float4 c[4];
+#pragma unroll
+    for (int u = 0; u < 4; u++) c[u] = A.cell_rec[min(b + u, max(e - 1, 0))];
+    for (int q = b; q < e; q += 4) {
+      float r2[4];
+      bool edge = false;
+#pragma unroll
+      for (int u = 0; u < 4; u++) {
+        r2[u] = q + u < e ? dist(c[u]) : fhi;
+        edge |= r2[u] >= flo && r2[u] < fhi;
+      }
+#pragma unroll
+      for (int u = 0; u < 4; u++) c[u] = A.cell_rec[min(q + 4 + u, e - 1)];
+      if (edge) {
+#pragma unroll
+        for (int u = 0; u < 4; u++)
+          if (r2[u] >= flo && r2[u] < fhi) r2[u] = exact(r2[u], q + u);
+      }
+#pragma unroll
+      for (int u = 0; u < 4; u++) take(r2[u], q + u);
+    }
+    __syncwarp();
+  }
+  // ---- the row, band by band
+  const int n = min(m, lcap);
+#pragma unroll
+  for (int b = 0; b < 10; b++) hist[32 * b] = 0;
+  unsigned code[9];
+#pragma unroll
+  for (int k = 0; k < 9; k++) code[k] = fr.code[k];
+  for (int e = 0; e < n; e++) {
+    const unsigned v = (unsigned)col[32 * e], c = v >> 16;
+    int b = c >= code[0];  // 0 inner, 1 below the first threshold, 2.. above it
+#pragma unroll
+    for (int k = 1; k < 9; k++) b += c > code[k];
+    hist[32 * b]++;
+    col[32 * e] = (int)(v & 0xffffu) | b << 16;
+  }
+  __syncwarp();
+  int run = 0, at0[10];
+  unsigned h[8];
+#pragma unroll
+  for (int b = 0; b < 10; b++) {
+    int before = 0, all = hist[32 * b];
+    if (SP > 1) {  // over the atom's lanes
+      all = 0;
+#pragma unroll
+      for (int o = 0; o < SP; o++) {
+        const int v = hist[32 * b + o - part];
+        all += v;
+        before += o < part ? v : 0;
+      }
+    }
+    at0[b] = run + before;
+    run += all;
+    if (b >= 1 && b < 9) h[b - 1] = min(run, 65535);  // entries not above threshold b - 1
+  }
+  __syncwarp();
+#pragma unroll
+  for (int b = 0; b < 10; b++) hist[32 * b] = at0[b];
+  if (SP > 1) {
+    int all = 0;
+#pragma unroll
+    for (int o = 0; o < SP; o++) all += __shfl_sync(FULL, m, (ln - part + o) & 31);
+    m = all;
+  }
+  if (act) {
+    for (int e = 0; e < n; e++) {
+      const int v = col[32 * e];
+      int* o = hist + 32 * (v >> 16);
+      const int at = *o;
+      *o = at + 1;
+      const int q = start[32 * (v >> 11 & 31)] + (v & 2047);
+      if (at < lcap) A.flist[(size_t)at * A.cap + i] = __float_as_int(A.cell_rec[q].w);
+    }
+    if (part == 0) {
+      A.ncut[i] = make_uint4(h[0] | h[1] << 16, h[2] | h[3] << 16, h[4] | h[5] << 16, h[6] | h[7] << 16);
+      A.nn[i] = m;
+      A.hnn[i] = m;
+      if (m > lcap) atomicOr(&A.st[s].status, ST_OVERFLOW);
+    }
+  }
+  const int mx = __reduce_max_sync(FULL, act ? m : 0);
+  if (ln == 0) atomicMax(&A.st[s].maxnn, mx);
+  __syncwarp();
+}
+
+// the rows of the systems flagged for a rebuild; M: ROWS_ATOMS a block
+template <int SP>
+__global__ void __launch_bounds__(32 * ROWS_WARPS, 4) k_list_rows(Arena A, BlockMap M) {
+  extern __shared__ __align__(16) unsigned char rows_sh[];
+  __shared__ RowsFrame f;
+  const int warp = threadIdx.x >> 5, ln = threadIdx.x & 31;
+  int* buf = reinterpret_cast<int*>(rows_sh + warp * rows_warp_bytes(A.lcap));
+  int fs = -1;  // the system whose frame is in f
+  rebuild_items<32 * ROWS_WARPS>(M.nblk * rows_rounds(SP), [&](int w) {
+      const int b = w % M.nblk;
+      return rebuild_block(A, M, b, true) && rows_fit(A.sys[M.sys[b]], A.lcap);
+    }, [&](int w) {
+      const int b = w % M.nblk, s = M.sys[b];
+      const SysDev& S = A.sys[s];
+      if (s != fs) {
+        __syncthreads();
+        if (threadIdx.x == 0) f = rows_frame(S);
+        fs = s;
+        __syncthreads();
+      }
+      const int p0 = M.first[b] + (w / M.nblk * ROWS_WARPS + warp) * rows_per_warp(SP);
+      if (p0 < M.end[b]) list_rows_warp<SP>(A, s, S, f, p0, M.end[b], buf, ln);
     });
 }
 
 // verlet_self / verlet_selfhalf (src/Neighbour.F90:676-811): O(N^2) over the
 // system in increasing index, keep j if rd <= (rcut+nb_dcut)^2.  Candidate
 // positions are staged through shared memory one BLOCK-wide tile at a time.
-__global__ void k_list_n2(Arena A, BlockMap M) {
+static __global__ void k_list_n2(Arena A, BlockMap M) {
   __shared__ double4 tile[BLOCK];
   rebuild_items(M.nblk, [&](int b) { return rebuild_block(A, M, b, false); }, [&](int b) {
     const int s = M.sys[b];
@@ -1230,13 +1519,14 @@ __global__ void k_list_n2(Arena A, BlockMap M) {
 
 // rebuild counters; in_graph marks the copy captured inside a conditional
 // node, whose executions are counted for the launch statistics
-__global__ void k_count_rebuild(Arena A, const int* sys, int nsys, int in_graph) {
+static __global__ void k_count_rebuild(Arena A, const int* sys, int nsys, int in_graph) {
   int k = blockIdx.x * blockDim.x + threadIdx.x;
   if (k < nsys && sys[k] >= 0 && A.st[sys[k]].rebuild) {
     SysState& st = A.st[sys[k]];
     st.nupd++;
     st.dmax = 0.0;
     for (int d = 0; d < 3; d++) st.box_b[d] = A.sys[sys[k]].L[d];
+    A.sys_b[sys[k]] = A.sys[sys[k]];  // box and grid of this list, for gemsgpu_get_list
   }
   if (in_graph && k == 0) atomicAdd(A.body_runs, 1ull);
 }
@@ -1343,7 +1633,7 @@ __global__ void k_thermo_sum(Arena A, BlockMap M) {
 // probability nu dt and takes v = th[0] / sqrt(m) r per coordinate, th[0]
 // the reference's sqrt(kB T / (3N)^2) (set_andersen, :1343-1364); the
 // uniform and the normals come from the thermostat's own Philox stream.
-__global__ void k_thermo_apply(Arena A, BlockMap M) {
+static __global__ void k_thermo_apply(Arena A, BlockMap M) {
   int s = blk_sys(M);
   if (s < 0) return;  // padding block of a fixed-capacity map
   const SysDev& S = A.sys[s];
@@ -1373,7 +1663,7 @@ __global__ void k_thermo_apply(Arena A, BlockMap M) {
 
 // kinetic tensor sum_i m v (x) v of each system (inq_pressure,
 // Inq_Properties.F90:529-573), into SysState::ktens
-__global__ void k_kin_tensor(Arena A, BlockMap M) {
+static __global__ void k_kin_tensor(Arena A, BlockMap M) {
   int s = blk_sys(M);
   if (s < 0) return;  // padding block of a fixed-capacity map
   int i = M.first[blockIdx.x] + threadIdx.x;
@@ -2611,7 +2901,7 @@ __device__ __forceinline__ void tsf_rslot_row(const Arena& A, int i, int m0, int
 }
 
 // the reverse slots of the Tersoff systems flagged for a rebuild
-__global__ void k_tsf_rslot(Arena A, BlockMap M) {
+static __global__ void k_tsf_rslot(Arena A, BlockMap M) {
   rebuild_items(M.nblk, [&](int b) {
       const int s = M.sys[b];
       return s >= 0 && A.st[s].rebuild && A.sys[s].ff == FF_TERSOFF;
@@ -2622,11 +2912,11 @@ __global__ void k_tsf_rslot(Arena A, BlockMap M) {
 }
 
 // interleaved [x1,y1,z1,...] staging <-> double4 arena slots
-__global__ void k_unpack3(const double* __restrict__ src, double4* __restrict__ dst, int n) {
+static __global__ void k_unpack3(const double* __restrict__ src, double4* __restrict__ dst, int n) {
   int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i < n) dst[i] = make_double4(src[3 * i], src[3 * i + 1], src[3 * i + 2], 0.0);
 }
-__global__ void k_pack3(const double4* __restrict__ src, double* __restrict__ dst, int n) {
+static __global__ void k_pack3(const double4* __restrict__ src, double* __restrict__ dst, int n) {
   int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i < n) {
     double4 v = src[i];
@@ -2637,7 +2927,7 @@ __global__ void k_pack3(const double4* __restrict__ src, double* __restrict__ ds
 }
 
 // velocity rescale of whole systems (replica exchange): v *= f[k]
-__global__ void k_scale_vel(Arena A, BlockMap M, const double* fac_by_sys) {
+static __global__ void k_scale_vel(Arena A, BlockMap M, const double* fac_by_sys) {
   int s = blk_sys(M);
   if (s < 0) return;  // padding block of a fixed-capacity map
   int i = M.first[blockIdx.x] + threadIdx.x;
@@ -2648,7 +2938,7 @@ __global__ void k_scale_vel(Arena A, BlockMap M, const double* fac_by_sys) {
   A.vel[i] = v;
 }
 
-__global__ void k_zero_force(Arena A, BlockMap M) {
+static __global__ void k_zero_force(Arena A, BlockMap M) {
   int i = M.first[blockIdx.x] + threadIdx.x;
   if (i < M.end[blockIdx.x]) A.force[i] = make_double4(0, 0, 0, 0);
 }
@@ -3043,7 +3333,7 @@ __device__ __forceinline__ void lkd_piston(const SysDev& S, SysState& st, const 
 // the pressure of the kicked velocities and the box's two half advances
 //   L_h = L (1 + dt/2 pvel / (Q V))^(1/3),  L' = L_h (1 + dt/2 pvel / (Q V_h))^(1/3)
 // (single-precision exponent 1./dd), which k_step_a applies to the atoms.
-__global__ void __launch_bounds__(BLOCK) k_lkd_a(Arena A, BlockMap M) {
+static __global__ void __launch_bounds__(BLOCK) k_lkd_a(Arena A, BlockMap M) {
   int s = blk_sys(M);
   if (s < 0) return;  // padding block of a fixed-capacity map
   SysDev& S = A.sys[s];
@@ -3112,7 +3402,7 @@ __global__ void __launch_bounds__(BLOCK) k_lkd_a(Arena A, BlockMap M) {
 // the reference, and the cell grid of the next rebuild re-planned for the
 // new lengths within the cells allocated.  The first step takes pistonf
 // from the virial of the initial interact and leaves pvel at 0.
-__global__ void k_lgf_sys(Arena A, const int* sys, int nsys) {
+static __global__ void k_lgf_sys(Arena A, const int* sys, int nsys) {
   const int k = blockIdx.x * blockDim.x + threadIdx.x;
   if (k >= nsys) return;
   const int s = sys[k];

@@ -72,11 +72,16 @@ constexpr int TEAM_BAR = 32;               // 128 B between the teams' counters
 constexpr int TEAM_TILE = 1024;            // candidates staged per cell in the team's list build
 constexpr unsigned TEAM_SPINS = 1u << 23;  // polls before a barrier gives up (seconds)
 
-// shared memory of the rebuild (and of Tersoff's bonds)
-__host__ __device__ constexpr size_t team_smem(int lcap, int ncell, bool warp_cells, size_t tsf) {
+// warps of a CTA that build lists (rows_fit systems): what 60 KB hold
+__host__ __device__ constexpr int team_row_warps(int lcap) {
+  const int w = (int)(60 * 1024 / rows_warp_bytes(lcap));
+  return w < 1 ? 1 : w > BLOCK / 32 ? BLOCK / 32 : w;
+}
+// shared memory of the rebuild (and of Tersoff's bonds); rows: rows_fit systems
+__host__ __device__ constexpr size_t team_smem(int lcap, int ncell, bool rows, size_t tsf) {
   const size_t scan = (size_t)(ncell + 1) * sizeof(int);
   const size_t list = ncell == 0 ? 0
-                      : warp_cells ? listw_smem<128>(lcap)
+                      : rows       ? team_row_warps(lcap) * rows_warp_bytes(lcap)
                                    : (size_t)TEAM_TILE * sizeof(float4) +
                                          (size_t)LIST_ATOMS * lcap * (sizeof(int) + sizeof(float));
   const size_t a = scan > list ? scan : list;
@@ -283,16 +288,18 @@ __device__ __noinline__ bool team_rebuild(const Arena& A, TeamCtl& c, int s, con
       sort_cell(A, start, n, ln);
     }
     if (!team_sync<RES>(c)) return false;
-    if (S.list_warp == 1) {
-      unsigned char* mine = dyn + (size_t)warp * listw_warp_bytes<128>(A.lcap);
-      float4* cf = reinterpret_cast<float4*>(mine);
-      int* boff = reinterpret_cast<int*>(cf + 128);
-      int* row = boff + 16;
-      float* rrow = reinterpret_cast<float*>(row + A.lcap);
-      for (int k = w0; k < S.ncell; k += wn) {
-        if (S.list_img) list_cells_w_item<true, 128>(A, s, S, S.cell_off + k, cf, boff, row, rrow);
-        else list_cells_w_item<false, 128>(A, s, S, S.cell_off + k, cf, boff, row, rrow);
-      }
+    if (rows_fit(S, A.lcap)) {
+      __shared__ RowsFrame f;
+      if (threadIdx.x == 0) f = rows_frame(S);
+      __syncthreads();
+      const int nw = team_row_warps(A.lcap), sp = rows_split(S.n, c.ncta * nw), per = rows_per_warp(sp);
+      int* buf = reinterpret_cast<int*>(dyn + (size_t)warp * rows_warp_bytes(A.lcap));
+      if (warp < nw)
+        for (int p0 = beg + (c.rank + warp * c.ncta) * per; p0 < end; p0 += c.ncta * nw * per) {
+          if (sp == 1) list_rows_warp<1>(A, s, S, f, p0, end, buf, ln);
+          else if (sp == 3) list_rows_warp<3>(A, s, S, f, p0, end, buf, ln);
+          else list_rows_warp<9>(A, s, S, f, p0, end, buf, ln);
+        }
     } else {
       // CTA per cell, or up to four CTAs where the team has more CTAs than cells
       float4* cf = reinterpret_cast<float4*>(dyn);
@@ -335,6 +342,7 @@ __device__ __noinline__ bool team_rebuild(const Arena& A, TeamCtl& c, int s, con
     st.nupd++;
     st.dmax = 0.0;
     for (int d = 0; d < 3; d++) st.box_b[d] = S.L[d];
+    if (c.rank == 0) A.sys_b[s] = S;
   }
   __syncthreads();
   return true;
@@ -895,5 +903,13 @@ __global__ void __launch_bounds__(BLOCK, MINB) k_team(const __grid_constant__ Ar
     }
   }
 }
+
+// the kernel of a kind for K lanes per atom, resident or arena form (team_inst.cu)
+const void* team_fn_0(int K, bool res);
+const void* team_fn_1(int K, bool res);
+const void* team_fn_2(int K, bool res);
+const void* team_fn_3(int K, bool res);
+const void* team_fn_4(int K, bool res);
+const void* team_fn_ts(bool mixed, int K);
 
 }  // namespace gg
