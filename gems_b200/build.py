@@ -17,7 +17,7 @@ OUT = os.path.join(HERE, "libgemsgpu.so")
 # (object, source, defines): the team kernels once per force-field kind
 UNITS = [("gemsgpu", "gemsgpu.cu", []), ("noalloc", "noalloc.cu", []), ("peaks", "peaks.cu", [])] + [
     ("team%d" % k, "team_inst.cu", ["-DTEAM_PART=%d" % k]) for k in range(6)]
-DEPS = [os.path.join(CSRC, f) for f in ("gemsgpu.cu", "noalloc.cu", "peaks.cu", "team_inst.cu", "kernels.cuh", "team.cuh",
+DEPS = [os.path.join(CSRC, f) for f in ("gemsgpu.cu", "noalloc.cu", "peaks.cu", "team_inst.cu", "kernels.cuh", "fp64.cuh", "team.cuh",
                                         "lbfgs.cuh", "neb.cuh", "common.cuh")] + [
     os.path.join(os.path.dirname(HERE), "include", "gemsgpu.h")]
 

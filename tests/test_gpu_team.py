@@ -178,3 +178,67 @@ def test_pair_functions_over_the_range(prec):
             ok[[-3, -1]] = False  # r = 5 is the cut-off: on which side is decided by the 2^-22 A grid
         assert np.abs(np.array(e) - eo)[ok].max() <= tol * np.abs(eo[ok]).max()
         assert np.abs(np.array(f) - fo)[ok].max() <= tol * np.abs(fo[ok]).max()
+
+
+def _noalloc(pos, L, pbc):
+    import ctypes
+    torch = pytest.importorskip("torch")
+    n = len(pos)
+    x = torch.tensor(pos.ravel(), dtype=torch.float64, device="cuda")
+    f = torch.full((3 * n,), np.nan, dtype=torch.float64, device="cuda")
+    e = torch.full((n,), np.nan, dtype=torch.float64, device="cuda")
+    L, ip = np.array(L, dtype=float), np.array(pbc, dtype=np.int32)
+    rc = gems.lib().gemsgpu_smatb_forces_noalloc(
+        ctypes.c_void_p(x.data_ptr()), n, int(ip.any()), L.ctypes.data_as(ctypes.POINTER(ctypes.c_double)),
+        ip.ctypes.data_as(ctypes.POINTER(ctypes.c_int)), *W.SMATB["Au"], ctypes.c_void_p(f.data_ptr()),
+        ctypes.c_void_p(e.data_ptr()), ctypes.c_void_p(torch.cuda.current_stream().cuda_stream))
+    assert rc == 0
+    return f.cpu().numpy().reshape(n, 3), e.cpu().numpy()
+
+
+@pytest.mark.parametrize("k", [0, 70])
+def test_noalloc_special_values(k):
+    """An atom at infinity (or beyond the squares' range) has no neighbours and
+    changes nobody else's forces; a NaN coordinate reaches every atom."""
+    pos = W.cluster(147, np.random.default_rng(5), check=False)
+    f0, e0 = _noalloc(np.delete(pos, k, 0), [400.0] * 3, [0, 0, 0])
+    for far in (np.inf, -np.inf, 1e39, 1e200):
+        pos[k] = far
+        f, e = _noalloc(pos, [400.0] * 3, [0, 0, 0])
+        assert (f[k] == 0.0).all() and e[k] == 0.0
+        assert np.abs(np.delete(f, k, 0) - f0).max() <= 1e-12 * np.abs(f0).max()
+        assert np.abs(np.delete(e, k) - e0).max() <= 1e-12 * np.abs(e0).max()
+    pos[k] = 0.0
+    pos[k, 1] = np.nan
+    f, e = _noalloc(pos, [400.0] * 3, [0, 0, 0])
+    assert np.isnan(f).all() and np.isnan(e).all()
+
+
+@pytest.mark.parametrize("n,box", [(1, None), (2, None), (31, None), (65, None), (2048, None), (2049, None), (4096, None),
+                                   (1372, (28.6, 28.6, 28.6)), (2916, (36.8, 36.8, 36.8)), (2916, (36.8, None, 36.8))])
+def test_noalloc_sizes(n, box):
+    """gemsgpu_smatb_forces_noalloc at the edges of its tiles and launch shapes,
+    clusters off the origin and periodic boxes with atoms outside them, against
+    the oracle: 1e-12 of the largest force (sums of 50 terms of 1e-15)."""
+    from oracle import oracle as O
+    rng = np.random.default_rng(n)
+    if box:
+        m = round((n / 4) ** (1 / 3))
+        pos, _ = lattice(FCC, 4.086, (m, m, m), rng, 0.08)
+        pos = pos + np.where(rng.random(pos.shape) < 0.1, 1, 0) * np.array([b or 0.0 for b in box])
+    else:
+        pos = W.cluster(n, rng, check=False) + np.array([300.0, -40.0, 7.0])
+    pbc = [1 if box and b else 0 for b in (box or (0, 0, 0))]
+    L = np.array([(b or 400.0) for b in (box or (0, 0, 0))], dtype=float)
+    o = O.System(np.mod(pos, np.where(pbc, L, 1e9)) if box else pos, W.MASS["Au"])
+    if box:
+        o.set_box(L, [bool(p) for p in pbc])
+    o.set_skin(0.1)
+    o.set_smatb(*W.SMATB["Au"])
+    o.interact()
+    f, e = _noalloc(pos, L, pbc)
+    if n == 1:  # no neighbour: rho = 0, no force
+        assert e[0] == 0.0 and (f == 0.0).all()
+        return
+    assert np.abs(f - o.force).max() <= 1e-12 * np.abs(o.force).max()
+    assert np.abs(e - o.epot_atoms).max() <= 1e-12 * np.abs(o.epot_atoms).max()
