@@ -160,6 +160,8 @@ struct gemsgpu_ctx {
   SysState* h_st = nullptr;
   double* stage = nullptr;      // 3 doubles per atom, host <-> device staging
   int64_t stage_cap = 0;
+  double* pin = nullptr;        // pinned host staging of small arrays (bounded, see XFER_PIN)
+  int64_t pin_cap = 0;          // doubles
   int64_t snap_cap = 0;
   double4* snap = nullptr;      // pos, vel, acel, force [, acel2, acel3, acel4]
   int snap_arrays = 0;
@@ -1045,7 +1047,7 @@ int launch_rebuild(gemsgpu_ctx* ctx, const std::vector<int>& ss, int in_graph = 
   if (ts) {
     k_tsf_rslot<<<rebuild_grid(ctx, ma.nblk), BLOCK, 0, st>>>(A, ma); ++ctx->launches;
   }
-  k_count_rebuild<<<((int)ss.size() + 255) / 256, 256, 0, st>>>(A, sa, (int)ss.size(), in_graph); ++ctx->launches;
+  k_count_rebuild<<<(int)ss.size(), 64, 0, st>>>(A, sa, in_graph); ++ctx->launches;
   CU(cudaGetLastError());
   return 0;
 }
@@ -1338,6 +1340,8 @@ bool team_clusters(gemsgpu_ctx* ctx, const std::vector<int>& ss, const void* fn,
 }
 
 // Assign the systems ss to teams; ctx->plan.use says whether the set runs there.
+constexpr int TEAM_RES_ATOMS = 2048;  // no larger system fits the resident form
+
 int team_plan(gemsgpu_ctx* ctx, const std::vector<int>& ss) {
   TeamPlan& P = ctx->plan;
   std::string key;
@@ -1416,7 +1420,7 @@ int team_plan(gemsgpu_ctx* ctx, const std::vector<int>& ss) {
     arena_ok = total <= (int64_t)occ * ctx->nsm;
   }
   std::vector<int> C;
-  const void* fn = ts || big > (arena_ok ? 640 : 2048) ? nullptr : team_fn(kind, K, true);
+  const void* fn = ts || big > (arena_ok ? 640 : TEAM_RES_ATOMS) ? nullptr : team_fn(kind, K, true);
   if (fn && team_clusters(ctx, ss, fn, kind, apb, scratch, C)) {
     P.fn = fn;
     std::vector<size_t> order(ss.size());  // the largest first
@@ -1536,23 +1540,30 @@ int ensure_list(gemsgpu_ctx* ctx, const std::vector<int>& ss) {
 // interact (src/Interaction.f90:135-241) for a set of systems, host-driven:
 // rebuild if flagged (heal overflow by growing the list), then forces.
 void settled(gemsgpu_ctx* ctx, const std::vector<int>& ss);
+int launch_reduce(gemsgpu_ctx* ctx, const std::vector<int>& ss);
 
-int interact_group(gemsgpu_ctx* ctx, const std::vector<int>& ss, bool sync_check) {
+// red: the caller wants the sums of launch_reduce next; *red says whether they
+// came with the states (one synchronisation for a small system's evaluation)
+int interact_group(gemsgpu_ctx* ctx, const std::vector<int>& ss, bool sync_check, bool* red = nullptr) {
   CHK(ensure_list(ctx, ss));
   bool built = false;  // h_st holds the states after a list update
   const int open = sync_check ? team_open(ctx, ss) : -1;
-  if (open > 0) {
+  int big = 0;
+  for (int s : ss) big = std::max(big, ctx->sys[s].n);
+  if (open > 0 && big <= TEAM_RES_ATOMS) {
     // small systems: lists and forces in one launch
     CHK(team_plan(ctx, ss));
     if (ctx->plan.use && ctx->plan.runs[0].cluster) {
       CHK(clear_status(ctx, ss));
       CHK(launch_team(ctx, open, 0));
+      if (red) CHK(launch_reduce(ctx, ss));
       CHK(read_states(ctx));
       bool over = false;
       for (int s : ss) over |= (ctx->h_st[s].status & ST_OVERFLOW) != 0;
       if (!over) {
         for (int s : ss) CHK(status_error(ctx, s, ctx->h_st[s].status));
         settled(ctx, ss);
+        if (red) *red = true;
         return 0;
       }
       built = true;  // a list overflowed: grown and built again below
@@ -1610,9 +1621,9 @@ int interact_group(gemsgpu_ctx* ctx, const std::vector<int>& ss, bool sync_check
 }
 
 // Epot, Ekin, max |F|^2 and the status of each system of ss (4 doubles per
-// system, in the order of ss): two grid-wide passes over the atom map
-int reduce_sys(gemsgpu_ctx* ctx, const std::vector<int>& ss, std::vector<double>& out) {
-  const int n = (int)ss.size();
+// system, in the order of ss): two grid-wide passes over the atom map, whose
+// results reduced() reads once the stream has been synchronised
+int launch_reduce(gemsgpu_ctx* ctx, const std::vector<int>& ss) {
   const int sc = ctx->scap;
   if (sc > ctx->h_red_cap) {
     if (ctx->h_red) cudaFreeHost(ctx->h_red);
@@ -1632,10 +1643,20 @@ int reduce_sys(gemsgpu_ctx* ctx, const std::vector<int>& ss, std::vector<double>
   }
   CU(cudaGetLastError());
   CU(cudaMemcpyAsync(ctx->h_red, ctx->d_red, 4 * sizeof(double) * sc, cudaMemcpyDeviceToHost, ctx->stream));
-  CU(cudaStreamSynchronize(ctx->stream));
+  return 0;
+}
+
+void reduced(const gemsgpu_ctx* ctx, const std::vector<int>& ss, std::vector<double>& out) {
+  const int n = (int)ss.size();
   out.assign(4 * (size_t)n, 0.0);
   for (int k = 0; k < n; k++)
     for (int q = 0; q < 4; q++) out[4 * (size_t)k + q] = ctx->h_red[4 * (size_t)ss[k] + q];
+}
+
+int reduce_sys(gemsgpu_ctx* ctx, const std::vector<int>& ss, std::vector<double>& out) {
+  CHK(launch_reduce(ctx, ss));
+  CU(cudaStreamSynchronize(ctx->stream));
+  reduced(ctx, ss, out);
   return 0;
 }
 
@@ -2104,6 +2125,141 @@ int d2h_xyz(gemsgpu_ctx* ctx, const double4* src, double* dst, int n) {
   return 0;
 }
 
+// Arrays of many systems between the host and the arena in one piece: arrays
+// up to XFER_SMALL doubles pass through a pinned buffer that the context keeps
+// (XFER_PIN doubles at most, 4 MB) and travel as one copy, larger ones travel
+// on their own, and one kernel repacks them all.  A copy and a repack per array
+// cost 5.8 us each way for a small one: 64 systems of 147 atoms took 1490 us
+// in and 1435 us out, @IN@ and @OUT@ us this way.  Above 64 KB a copy by the
+// processor takes longer than the copy engine's own start.
+constexpr int64_t XFER_SMALL = 8192, XFER_PIN = 1 << 19;
+
+struct Xfer {
+  struct Item {
+    int s, a;         // system, array
+    double* host;
+    int64_t len, at;  // doubles, place in the staging buffer
+    bool small;
+  };
+  std::vector<Item> items;
+  int64_t head = 0, nsmall = 0;  // the table and the small arrays lead the buffer
+  int s0 = 0;
+  XferAt one;  // a single system's table travels with the launch: head is 0
+};
+
+int ensure_pin(gemsgpu_ctx* ctx, int64_t n) {
+  CU(cudaStreamSynchronize(ctx->stream));  // nothing reads it any more
+  if (ctx->pin_cap >= n) return 0;
+  int64_t cap = 4096;
+  while (cap < n) cap *= 2;
+  if (ctx->pin) CU(cudaFreeHost(ctx->pin));
+  ctx->pin = nullptr;
+  ctx->pin_cap = 0;
+  CU(cudaMallocHost((void**)&ctx->pin, cap * sizeof(double)));
+  ctx->pin_cap = cap;
+  return 0;
+}
+
+// lay out host[a], array a (XA_*) of each system of ss (or null), and write the
+// table of their places at the head of the pinned buffer
+int xfer_plan(gemsgpu_ctx* ctx, const std::vector<int>& ss, const double* const* const host[XA_N], Xfer& x) {
+  const auto ends = std::minmax_element(ss.begin(), ss.end());
+  x.s0 = *ends.first;
+  x.head = ss.size() > 1 ? (int64_t)(*ends.second - x.s0 + 1) * XA_N : 0;
+  for (int a = 0; a < XA_N; a++)
+    for (size_t k = 0; host[a] && k < ss.size(); k++) {
+      if (!host[a][k]) continue;
+      const int64_t len = (int64_t)xa_width(a) * ctx->sys[ss[k]].n;
+      const bool small = len <= XFER_SMALL && x.nsmall + len <= XFER_PIN;
+      x.items.push_back({ss[k], a, const_cast<double*>(host[a][k]), len, small ? x.head + x.nsmall : 0, small});
+      if (small) x.nsmall += len;
+    }
+  int64_t total = x.head + x.nsmall;
+  for (Xfer::Item& t : x.items)
+    if (!t.small) {
+      t.at = total;
+      total += t.len;
+    }
+  if (x.head + x.nsmall) CHK(ensure_pin(ctx, x.head + x.nsmall));
+  CHK(ensure_stage(ctx, (total + 2) / 3));
+  long long* tab = x.head ? (long long*)ctx->pin : x.one.at;
+  std::fill(tab, tab + std::max<int64_t>(x.head, XA_N), XFER_NONE);
+  for (const Xfer::Item& t : x.items)  // so that the arena index finds the atom
+    tab[(t.s - x.s0) * XA_N + t.a] = t.at - (long long)xa_width(t.a) * ctx->sys[t.s].off;
+  return 0;
+}
+
+int xfer_kernel(gemsgpu_ctx* ctx, const std::vector<int>& ss, const Xfer& x, bool in) {
+  BlockMap m;
+  CHK(get_map(ctx, ss, BLOCK, 0, &m));
+  if (m.nblk > 0) {
+    if (in) k_xfer<true><<<m.nblk, BLOCK, 0, ctx->stream>>>(ctx->A, m, ctx->stage, x.s0, x.one, !x.head);
+    else k_xfer<false><<<m.nblk, BLOCK, 0, ctx->stream>>>(ctx->A, m, ctx->stage, x.s0, x.one, !x.head);
+    ++ctx->launches;
+  }
+  CU(cudaGetLastError());
+  return 0;
+}
+
+// positions (with their fixed-point copies) and velocities of ss, synchronised
+int xfer_in(gemsgpu_ctx* ctx, const std::vector<int>& ss, const double* const* pos, const double* const* vel) {
+  const double* const* host[XA_N] = {pos, vel, nullptr, nullptr};
+  Xfer x;
+  CHK(xfer_plan(ctx, ss, host, x));
+  if (x.items.empty()) return 0;
+  for (const Xfer::Item& t : x.items)
+    if (t.small) std::memcpy(ctx->pin + t.at, t.host, t.len * sizeof(double));
+  if (x.head + x.nsmall)
+    CU(cudaMemcpyAsync(ctx->stage, ctx->pin, (x.head + x.nsmall) * sizeof(double), cudaMemcpyHostToDevice, ctx->stream));
+  for (const Xfer::Item& t : x.items)
+    if (!t.small)
+      CU(cudaMemcpyAsync(ctx->stage + t.at, t.host, t.len * sizeof(double), cudaMemcpyHostToDevice, ctx->stream));
+  CHK(xfer_kernel(ctx, ss, x, true));
+  CU(cudaStreamSynchronize(ctx->stream));
+  return 0;
+}
+
+// arrays of ss to the host; `red`: and the sums of launch_reduce
+int xfer_out(gemsgpu_ctx* ctx, const std::vector<int>& ss, const double* const* const host[XA_N],
+             std::vector<double>* red = nullptr) {
+  Xfer x;
+  CHK(xfer_plan(ctx, ss, host, x));
+  if (!x.items.empty()) {
+    if (x.head)
+      CU(cudaMemcpyAsync(ctx->stage, ctx->pin, x.head * sizeof(double), cudaMemcpyHostToDevice, ctx->stream));
+    CHK(xfer_kernel(ctx, ss, x, false));
+    if (x.nsmall)
+      CU(cudaMemcpyAsync(ctx->pin + x.head, ctx->stage + x.head, x.nsmall * sizeof(double), cudaMemcpyDeviceToHost,
+                         ctx->stream));
+    for (const Xfer::Item& t : x.items)
+      if (!t.small)
+        CU(cudaMemcpyAsync(t.host, ctx->stage + t.at, t.len * sizeof(double), cudaMemcpyDeviceToHost, ctx->stream));
+  }
+  if (red) CHK(launch_reduce(ctx, ss));
+  CU(cudaStreamSynchronize(ctx->stream));
+  if (red) reduced(ctx, ss, *red);
+  for (const Xfer::Item& t : x.items)
+    if (t.small) std::memcpy(t.host, ctx->pin + t.at, t.len * sizeof(double));
+  return 0;
+}
+
+// the SysDev records of ss in one copy (their parameter tables unchanged)
+int push_devs(gemsgpu_ctx* ctx, const std::vector<int>& ss) {
+  constexpr int W = sizeof(SysDev) / sizeof(double);
+  static_assert(sizeof(SysDev) % sizeof(double) == 0, "SysDev is copied in words of 8 bytes");
+  const int64_t n = (int64_t)ss.size() * (W + 1);
+  CHK(ensure_pin(ctx, n));
+  CHK(ensure_stage(ctx, (n + 2) / 3));
+  for (size_t k = 0; k < ss.size(); k++) {
+    std::memcpy(ctx->pin + k * (W + 1), &ctx->sys[ss[k]].d, sizeof(SysDev));
+    ((long long*)ctx->pin)[k * (W + 1) + W] = ss[k];
+  }
+  CU(cudaMemcpyAsync(ctx->stage, ctx->pin, n * sizeof(double), cudaMemcpyHostToDevice, ctx->stream));
+  k_put_devs<<<(int)ss.size(), 64, 0, ctx->stream>>>(ctx->A, (const long long*)ctx->stage); ++ctx->launches;
+  CU(cudaGetLastError());
+  return 0;
+}
+
 void copy_interleaved_to_d4(const double* src, std::vector<double4>& dst, int n) {
   dst.resize(n);
   for (int i = 0; i < n; i++) dst[i] = make_double4(src[3 * i], src[3 * i + 1], src[3 * i + 2], 0.0);
@@ -2220,7 +2376,7 @@ int pool_rebuild(gemsgpu_pool* P, int in_graph) {
   if (P->ff == FF_TERSOFF) {
     k_tsf_rslot<<<rebuild_grid(ctx, ma.nblk), BLOCK, 0, st>>>(A, ma); ++ctx->launches;
   }
-  k_count_rebuild<<<(ns + 255) / 256, 256, 0, st>>>(A, P->dsys, ns, in_graph); ++ctx->launches;
+  k_count_rebuild<<<ns, 64, 0, st>>>(A, P->dsys, in_graph); ++ctx->launches;
   CU(cudaGetLastError());
   return 0;
 }
@@ -2470,6 +2626,7 @@ int gemsgpu_destroy(gemsgpu_ctx* ctx) {
   if (ctx->h_red) cudaFreeHost(ctx->h_red);
   if (ctx->h_st) cudaFreeHost(ctx->h_st);
   if (ctx->stage) cudaFree(ctx->stage);
+  if (ctx->pin) cudaFreeHost(ctx->pin);
   for (auto st : ctx->side) cudaStreamDestroy(st);
   for (auto ev : ctx->side_done) cudaEventDestroy(ev);
   if (ctx->side_go) cudaEventDestroy(ctx->side_go);
@@ -2598,11 +2755,7 @@ int gemsgpu_set_positions(gemsgpu_ctx* ctx, int sys, const double* pos) {
   CHK(check_sys(ctx, sys));
   if (!pos) return fail(ctx, GEMSGPU_ERR_ARG, "set_positions: NULL");
   SysHost& h = ctx->sys[sys];
-  CHK(h2d_xyz(ctx, pos, ctx->A.pos + h.off, h.n));
-  BlockMap m;
-  CHK(get_map(ctx, {sys}, BLOCK, 0, &m));
-  k_refresh_fx<<<m.nblk, BLOCK, 0, ctx->stream>>>(ctx->A, m); ++ctx->launches;
-  CU(cudaStreamSynchronize(ctx->stream));
+  CHK(xfer_in(ctx, {sys}, &pos, nullptr));
   h.pos_dirty = true;
   h.has_forces = false;
   return 0;
@@ -2635,16 +2788,10 @@ static int get_d4(gemsgpu_ctx* ctx, const SysHost& h, const double4* src, double
 int gemsgpu_download(gemsgpu_ctx* ctx, int sys, double* pos, double* vel, double* force,
                      double* epot_atoms) {
   CHK(check_sys(ctx, sys));
-  const SysHost& h = ctx->sys[sys];
-  if (pos) CHK(get_d4(ctx, h, ctx->A.pos, pos));
-  if (vel) CHK(get_d4(ctx, h, ctx->A.vel, vel));
-  if (force) CHK(get_d4(ctx, h, ctx->A.force, force));
-  if (epot_atoms) {
-    CU(cudaMemcpyAsync(epot_atoms, ctx->A.epot + h.off, h.n * sizeof(double), cudaMemcpyDeviceToHost,
-                       ctx->stream));
-    CU(cudaStreamSynchronize(ctx->stream));
-  }
-  return 0;
+  const double* const p[XA_N] = {pos, vel, force, epot_atoms};
+  const double* const* host[XA_N];
+  for (int a = 0; a < XA_N; a++) host[a] = p[a] ? &p[a] : nullptr;
+  return xfer_out(ctx, {sys}, host);
 }
 
 int gemsgpu_download_acel(gemsgpu_ctx* ctx, int sys, double* acel) {
@@ -2826,10 +2973,12 @@ int gemsgpu_forces(gemsgpu_ctx* ctx, int sys, double* epot, int* rebuilt) {
     CHK(read_states(ctx));
     before = ctx->h_st[sys].nupd;
   }
-  CHK(interact_group(ctx, {sys}, true));
+  bool red = false;
+  CHK(interact_group(ctx, {sys}, true, epot || rebuilt ? &red : nullptr));
   if (epot || rebuilt) {
     std::vector<double> r;
-    CHK(reduce_sys(ctx, {sys}, r));
+    if (red) reduced(ctx, {sys}, r);
+    else CHK(reduce_sys(ctx, {sys}, r));
     if (epot) *epot = r[0];
     if (rebuilt) {
       CHK(read_states(ctx));
@@ -3072,16 +3221,8 @@ int gemsgpu_set_fire(gemsgpu_ctx* ctx, int sys, double dt0, double dtmax) {
   h.d.fire_fmax = 0.0;
   h.d.fire_maxit = 0x7fffffff;
   CHK(push_sys(ctx, sys));
-  SysState z{};
-  CHK(read_states(ctx));
-  z.nupd = ctx->h_st[sys].nupd;
-  z.fire_dt = dt0;
-  z.fire_alpha = 0.1;
-  CU(cudaMemcpyAsync(ctx->A.st + sys, &z, sizeof(z), cudaMemcpyHostToDevice, ctx->stream));
-  std::vector<double4> zero(h.n, make_double4(0, 0, 0, 0));
-  CU(cudaMemcpyAsync(ctx->A.vel + h.off, zero.data(), h.n * sizeof(double4), cudaMemcpyHostToDevice,
-                     ctx->stream));
-  CU(cudaStreamSynchronize(ctx->stream));
+  k_fire_reset<<<(h.n + 255) / 256, 256, 0, ctx->stream>>>(ctx->A, sys, dt0); ++ctx->launches;
+  CU(cudaGetLastError());
   invalidate(ctx);
   return 0;
 }
@@ -3537,20 +3678,21 @@ int gemsgpu_batch_fire(gemsgpu_ctx* ctx, const int* sys, int nsys, double fmax, 
     if (h.d.integ != IT_FIRE) return fail(ctx, GEMSGPU_ERR_STATE, "system %d is not set up for FIRE", s);
     h.d.fire_fmax = fmax;
     h.d.fire_maxit = maxit;
-    CHK(push_sys(ctx, s));
+    if (h.box_live) CHK(live_box(ctx, s, h.d.L));
+    derive(ctx, h);
+    CHK(alloc_cells(ctx, h));
   }
+  CHK(push_devs(ctx, ss));
   invalidate(ctx);
   // converged systems freeze on the device; poll between chunks
   CHK(interact_group(ctx, ss, true));
   {
-    std::vector<double> r;
-    CHK(reduce_sys(ctx, ss, r));
-    CHK(read_states(ctx));
-    for (size_t k = 0; k < ss.size(); k++) {
-      SysState st = ctx->h_st[ss[k]];
-      st.fire_done = std::sqrt(r[4 * k + 2]) * UI_EV < fmax ? 1 : 0;
-      CU(cudaMemcpyAsync(ctx->A.st + ss[k], &st, sizeof(st), cudaMemcpyHostToDevice, ctx->stream));
-    }
+    const int* sa;
+    CHK(launch_reduce(ctx, ss));
+    CHK(sys_array(ctx, ss, &sa));
+    k_fire_done<<<((int)ss.size() + 255) / 256, 256, 0, ctx->stream>>>(ctx->A, sa, (int)ss.size(), ctx->d_red, fmax);
+    ++ctx->launches;
+    CU(cudaGetLastError());
   }
   int total = 0;
   bool uniform = true;
@@ -3645,44 +3787,17 @@ int gemsgpu_batch_energy(gemsgpu_ctx* ctx, const int* sys, int nsys, double* epo
   return 0;
 }
 
-// Host <-> device state of many systems in one call: every copy and repack
-// is queued on the context's stream and the call synchronises once (the
-// per-system calls synchronise each time).  The staging buffer holds two
-// regions of 3 doubles per atom of the whole set, so no copy waits for
-// another's repack.
+// Host <-> device state of many systems in one call, with one synchronisation.
 int gemsgpu_batch_set_state(gemsgpu_ctx* ctx, const int* sys, int nsys, const double* const* pos,
                             const double* const* vel) {
   std::vector<int> ss;
   CHK(sys_list(ctx, sys, nsys, ss));
   if (!pos && !vel) return fail(ctx, GEMSGPU_ERR_ARG, "batch_set_state: nothing to set");
   cudaSetDevice(ctx->device);
-  int64_t total = 0;
-  for (int s : ss) total += ctx->sys[s].n;
-  CHK(ensure_stage(ctx, 2 * total));
-  int64_t o = 0;
+  CHK(xfer_in(ctx, ss, pos, vel));
   std::vector<int> moved;
-  for (int k = 0; k < nsys; k++) {
-    SysHost& h = ctx->sys[ss[k]];
-    double* sp = ctx->stage + 3 * o;
-    double* sv = ctx->stage + 3 * (total + o);
-    if (pos && pos[k]) {
-      CU(cudaMemcpyAsync(sp, pos[k], (size_t)3 * h.n * sizeof(double), cudaMemcpyHostToDevice, ctx->stream));
-      k_unpack3<<<(h.n + 255) / 256, 256, 0, ctx->stream>>>(sp, ctx->A.pos + h.off, h.n); ++ctx->launches;
-      moved.push_back(ss[k]);
-    }
-    if (vel && vel[k]) {
-      CU(cudaMemcpyAsync(sv, vel[k], (size_t)3 * h.n * sizeof(double), cudaMemcpyHostToDevice, ctx->stream));
-      k_unpack3<<<(h.n + 255) / 256, 256, 0, ctx->stream>>>(sv, ctx->A.vel + h.off, h.n); ++ctx->launches;
-    }
-    o += h.n;
-  }
-  if (!moved.empty()) {
-    BlockMap m;
-    CHK(get_map(ctx, moved, BLOCK, 0, &m));
-    k_refresh_fx<<<m.nblk, BLOCK, 0, ctx->stream>>>(ctx->A, m); ++ctx->launches;
-  }
-  CU(cudaGetLastError());
-  CU(cudaStreamSynchronize(ctx->stream));
+  for (int k = 0; pos && k < nsys; k++)
+    if (pos[k]) moved.push_back(ss[k]);
   for (int s : moved) {
     ctx->sys[s].pos_dirty = true;
     ctx->sys[s].has_forces = false;
@@ -3695,35 +3810,15 @@ int gemsgpu_batch_get_state(gemsgpu_ctx* ctx, const int* sys, int nsys, double* 
   std::vector<int> ss;
   CHK(sys_list(ctx, sys, nsys, ss));
   cudaSetDevice(ctx->device);
-  int64_t total = 0;
-  for (int s : ss) total += ctx->sys[s].n;
-  CHK(ensure_stage(ctx, 2 * total));
-  int64_t o = 0;
-  for (int k = 0; k < nsys; k++) {
-    const SysHost& h = ctx->sys[ss[k]];
-    double* sp = ctx->stage + 3 * o;
-    double* sv = ctx->stage + 3 * (total + o);
-    if (pos && pos[k]) {
-      k_pack3<<<(h.n + 255) / 256, 256, 0, ctx->stream>>>(ctx->A.pos + h.off, sp, h.n); ++ctx->launches;
-      CU(cudaMemcpyAsync(pos[k], sp, (size_t)3 * h.n * sizeof(double), cudaMemcpyDeviceToHost, ctx->stream));
-    }
-    if (vel && vel[k]) {
-      k_pack3<<<(h.n + 255) / 256, 256, 0, ctx->stream>>>(ctx->A.vel + h.off, sv, h.n); ++ctx->launches;
-      CU(cudaMemcpyAsync(vel[k], sv, (size_t)3 * h.n * sizeof(double), cudaMemcpyDeviceToHost, ctx->stream));
-    }
-    o += h.n;
-  }
-  CU(cudaGetLastError());
+  const double* const* host[XA_N] = {pos, vel, nullptr, nullptr};
+  std::vector<double> r;
+  CHK(xfer_out(ctx, ss, host, epot_ev || ekin_ev || temp ? &r : nullptr));
   if (epot_ev || ekin_ev || temp) {
-    std::vector<double> r;
-    CHK(reduce_sys(ctx, ss, r));  // synchronises the stream
     for (int k = 0; k < nsys; k++) {
       if (epot_ev) epot_ev[k] = r[4 * k] * UI_EV;
       if (ekin_ev) ekin_ev[k] = r[4 * k + 1] * UI_EV;
       if (temp) temp[k] = 2.0 * r[4 * k + 1] / (kB_ui * (3.0 * ctx->sys[ss[k]].n));
     }
-  } else {
-    CU(cudaStreamSynchronize(ctx->stream));
   }
   return 0;
 }
@@ -3774,7 +3869,7 @@ static int autotune_set(gemsgpu_ctx* ctx, const std::vector<int>& ss, int reps, 
   cudaEvent_t e0, e1;
   CU(cudaEventCreate(&e0));
   CU(cudaEventCreate(&e1));
-  double best = 1e30;
+  double best = 1e30, took = 0.0;
   std::pair<int, int> pick = {h0.lanes, h0.variant};
   for (auto c : cand) {
     for (int s : ss) {
@@ -3785,7 +3880,8 @@ static int autotune_set(gemsgpu_ctx* ctx, const std::vector<int>& ss, int reps, 
     // will run it
     invalidate(ctx);
     CHK(team_plan(ctx, ss));
-    const bool team = ctx->plan.use;
+    // (without an integrator only the resident form evaluates)
+    const bool team = ctx->plan.use && (ctx->plan.runs[0].cluster || h0.d.integ != IT_NONE);
     auto once = [&]() -> int { return team ? launch_team(ctx, TF_FORCE, 0) : launch_forces(ctx, ss); };
     CHK(once());  // warm-up (and map creation)
     CU(cudaEventRecord(e0, ctx->stream));
@@ -3794,9 +3890,11 @@ static int autotune_set(gemsgpu_ctx* ctx, const std::vector<int>& ss, int reps, 
     CU(cudaEventSynchronize(e1));
     float ms;
     CU(cudaEventElapsedTime(&ms, e0, e1));
-    if (!team) ms += 0.012f * reps;  // the step's other launches, which a team does not have
-    if (ms / reps < best) {
-      best = ms / reps;
+    // a step's other launches, which a team does not have
+    const float rank = ms / reps + (team ? 0.0f : 0.012f);
+    if (rank < best) {
+      best = rank;
+      took = ms / reps;
       pick = c;
     }
   }
@@ -3809,7 +3907,7 @@ static int autotune_set(gemsgpu_ctx* ctx, const std::vector<int>& ss, int reps, 
   invalidate(ctx);
   if (lanes_out) *lanes_out = pick.first;
   if (variant_out) *variant_out = pick.second;
-  if (best_ms) *best_ms = best;
+  if (best_ms) *best_ms = took;
   return 0;
 }
 

@@ -501,42 +501,52 @@ __device__ __forceinline__ bool ref_list_block(const Arena& A, const BlockMap& M
 }
 
 // atom i at place p of the cell order: its position, and in single precision
-// (with the atom's id) for the list kernel's filter
-__device__ __forceinline__ void put_cell(const Arena& A, int p, int i) {
+// (with the atom's id) for the filter of k_list_rows (rec)
+__device__ __forceinline__ void put_cell(const Arena& A, int p, int i, bool rec) {
   const double4 x = A.pos[i];
   A.cell_pos[p] = x;
-  A.cell_rec[p] = make_float4((float)x.x, (float)x.y, (float)x.z, __int_as_float(i));
+  if (rec) A.cell_rec[p] = make_float4((float)x.x, (float)x.y, (float)x.z, __int_as_float(i));
 }
 
-// one warp orders the n atoms of the cell whose atoms start at `start`
-__device__ __forceinline__ void sort_cell(const Arena& A, int start, int n, int ln) {
+// atoms of one cell, at most 32 R: each lane ranks its R (the entries greater
+// than its own; empty slots, -1, are greater than none) and places them
+template <int R>
+__device__ __forceinline__ void rank_cell(const Arena& A, int start, int n, int ln, bool rec) {
   int* a = A.cell_atoms + start;
+  int v[R], r[R] = {};
+#pragma unroll
+  for (int u = 0; u < R; u++) v[u] = ln + 32 * u < n ? a[ln + 32 * u] : -1;
+#pragma unroll
+  for (int t = 0; t < R; t++)
+    for (int k = 0; k < min(n - 32 * t, 32); k++) {
+      const int w = __shfl_sync(0xffffffffu, v[t], k);
+#pragma unroll
+      for (int u = 0; u < R; u++) r[u] += w > v[u];
+    }
+  __syncwarp();
+#pragma unroll
+  for (int u = 0; u < R; u++)
+    if (ln + 32 * u < n) {
+      a[r[u]] = v[u];
+      put_cell(A, start + r[u], v[u], rec);
+    }
+}
+
+// one warp orders the n atoms of the cell whose atoms start at `start`; cells
+// of more than 64 atoms occur where a moving box leaves atoms outside its grid
+// (lane 0 alone took 50 us for one: 32000 atoms under a piston)
+template <int RMAX>
+__device__ __forceinline__ void sort_cell(const Arena& A, int start, int n, int ln, bool rec) {
   if (n <= 64) {
-    int v0 = ln < n ? a[ln] : -1;
-    int v1 = ln + 32 < n ? a[ln + 32] : -1;
-    int r0 = 0, r1 = 0;
-    // rank = entries greater than mine; empty slots (-1) are greater than none
-    for (int k = 0; k < min(n, 32); k++) {
-      const int w0 = __shfl_sync(0xffffffffu, v0, k);
-      r0 += w0 > v0;
-      r1 += w0 > v1;
-    }
-    for (int k = 0; k < n - 32; k++) {
-      const int w1 = __shfl_sync(0xffffffffu, v1, k);
-      r0 += w1 > v0;
-      r1 += w1 > v1;
-    }
-    __syncwarp();
-    // each lane places its own atoms (id and position) at their ranks
-    if (ln < n) {
-      a[r0] = v0;
-      put_cell(A, start + r0, v0);
-    }
-    if (ln + 32 < n) {
-      a[r1] = v1;
-      put_cell(A, start + r1, v1);
-    }
-  } else if (ln == 0) {
+    rank_cell<2>(A, start, n, ln, rec);
+    return;
+  }
+  if (RMAX > 2 && n <= 32 * RMAX) {
+    rank_cell<RMAX>(A, start, n, ln, rec);
+    return;
+  }
+  int* a = A.cell_atoms + start;
+  if (ln == 0)
     for (int x = 1; x < n; x++) {
       int v = a[x];
       int y = x - 1;
@@ -546,18 +556,19 @@ __device__ __forceinline__ void sort_cell(const Arena& A, int start, int n, int 
       }
       a[y + 1] = v;
     }
-    for (int x = 0; x < n; x++) put_cell(A, start + x, a[x]);  // the lane's own writes
-  }
+  __syncwarp();
+  for (int x = ln; x < n; x += 32) put_cell(A, start + x, a[x], rec);
 }
 
 static __global__ void k_sort_cells(Arena A, BlockMap C) {
   rebuild_items(C.nblk, [&](int b) { return rebuild_block(A, C, b, true); }, [&](int b) {
     const int warp = threadIdx.x >> 5, ln = threadIdx.x & 31;
     const int first = C.first[b], end = C.end[b];
+    const bool rec = rows_fit(A.sys[C.sys[b]], A.lcap);
     for (int c = first + warp; c < end; c += BLOCK / 32) {  // C: 8 cells per block
       const int start = A.chunk_sum[c >> 8] + A.cell_loc[c];
       if (ln == 0) A.cell_start[c] = start;
-      sort_cell(A, start, A.cell_n[c], ln);
+      sort_cell<8>(A, start, A.cell_n[c], ln, rec);
     }
     });
 }
@@ -1464,16 +1475,22 @@ static __global__ void k_list_n2(Arena A, BlockMap M) {
 
 // rebuild counters; in_graph marks the copy captured inside a conditional
 // node, whose executions are counted for the launch statistics
-static __global__ void k_count_rebuild(Arena A, const int* sys, int nsys, int in_graph) {
-  int k = blockIdx.x * blockDim.x + threadIdx.x;
-  if (k < nsys && sys[k] >= 0 && A.st[sys[k]].rebuild) {
-    SysState& st = A.st[sys[k]];
-    st.nupd++;
-    st.dmax = 0.0;
-    for (int d = 0; d < 3; d++) st.box_b[d] = A.sys[sys[k]].L[d];
-    A.sys_b[sys[k]] = A.sys[sys[k]];  // box and grid of this list, for gemsgpu_get_list
+// one block per system
+static __global__ void k_count_rebuild(Arena A, const int* sys, int in_graph) {
+  const int s = sys[blockIdx.x];
+  if (s >= 0 && A.st[s].rebuild) {
+    if (threadIdx.x == 0) {
+      SysState& st = A.st[s];
+      st.nupd++;
+      st.dmax = 0.0;
+      for (int d = 0; d < 3; d++) st.box_b[d] = A.sys[s].L[d];
+    }
+    // box and grid of this list, for gemsgpu_get_list
+    const long long* src = (const long long*)(A.sys + s);
+    long long* dst = (long long*)(A.sys_b + s);
+    for (int k = threadIdx.x; k < (int)(sizeof(SysDev) / 8); k += blockDim.x) dst[k] = src[k];
   }
-  if (in_graph && k == 0) atomicAdd(A.body_runs, 1ull);
+  if (in_graph && blockIdx.x == 0 && threadIdx.x == 0) atomicAdd(A.body_runs, 1ull);
 }
 
 // ------------------------------------------------------------------ reductions
@@ -2833,6 +2850,75 @@ static __global__ void k_pack3(const double4* __restrict__ src, double* __restri
     dst[3 * i + 1] = v.y;
     dst[3 * i + 2] = v.z;
   }
+}
+
+// Arrays of many systems between the host's staging buffer (a table of their
+// places, then xyz interleaved) and the arena, all systems in one launch.
+// at[a] + width * (arena index) finds the atom; XFER_NONE: not transferred.
+enum { XA_POS, XA_VEL, XA_FORCE, XA_EPOT, XA_N };
+constexpr long long XFER_NONE = -(1LL << 62);
+constexpr int xa_width(int a) { return a == XA_EPOT ? 1 : 3; }
+struct XferAt {
+  long long at[XA_N];
+};
+template <bool IN>
+static __global__ void k_xfer(Arena A, BlockMap M, double* stage, int s0, XferAt one, bool single) {
+  const int s = blk_sys(M);
+  if (s < 0) return;  // padding block of a fixed-capacity map
+  const int i = M.first[blockIdx.x] + threadIdx.x;
+  if (i >= M.end[blockIdx.x]) return;
+  const XferAt t = single ? one : ((const XferAt*)stage)[s - s0];
+  const long long* at = t.at;
+  double4* const arr[3] = {A.pos, A.vel, A.force};
+#pragma unroll
+  for (int a = 0; a < (IN ? 2 : 3); a++) {
+    if (at[a] == XFER_NONE) continue;
+    double* b = stage + (at[a] + 3LL * i);
+    if constexpr (IN) {
+      const double4 v = make_double4(b[0], b[1], b[2], 0.0);
+      arr[a][i] = v;
+      if (a == XA_POS) {
+        int bad = 0;
+        write_fx(A.fxp, A.sys[s], i, v, A.type[i], bad);
+        if (bad) atomicOr(&A.st[s].status, ST_LOST);
+      }
+    } else {
+      const double4 v = arr[a][i];
+      b[0] = v.x;
+      b[1] = v.y;
+      b[2] = v.z;
+    }
+  }
+  if (!IN && at[XA_EPOT] != XFER_NONE) stage[at[XA_EPOT] + i] = A.epot[i];
+}
+
+// records of systems: W words of SysDev and the system's index
+static __global__ void k_put_devs(Arena A, const long long* __restrict__ src) {
+  constexpr int W = sizeof(SysDev) / 8;
+  const long long* r = src + (size_t)blockIdx.x * (W + 1);
+  long long* d = (long long*)(A.sys + r[W]);
+  for (int k = threadIdx.x; k < W; k += blockDim.x) d[k] = r[k];
+}
+
+// FIRE's start: zero velocities and a fresh state that keeps the build count
+static __global__ void k_fire_reset(Arena A, int s, double dt0) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  const SysDev& S = A.sys[s];
+  if (i < S.n) A.vel[S.off + i] = make_double4(0.0, 0.0, 0.0, 0.0);
+  if (i) return;
+  const int64_t nupd = A.st[s].nupd;
+  SysState z{};
+  z.nupd = nupd;
+  z.fire_dt = dt0;
+  z.fire_alpha = 0.1;
+  A.st[s] = z;
+}
+
+// systems whose largest force (red: k_sys_reduce's results) is below fmax eV/A
+// are done before their first iteration
+static __global__ void k_fire_done(Arena A, const int* __restrict__ ss, int n, const double* __restrict__ red, double fmax) {
+  const int k = blockIdx.x * blockDim.x + threadIdx.x;
+  if (k < n) A.st[ss[k]].fire_done = sqrt(red[4 * (size_t)ss[k] + 2]) * c_ui_ev() < fmax ? 1 : 0;
 }
 
 // velocity rescale of whole systems (replica exchange): v *= f[k]

@@ -285,7 +285,7 @@ __device__ __noinline__ bool team_rebuild(const Arena& A, TeamCtl& c, int s, con
         A.cell_n[S.cell_off + k] = n;
         A.cell_count[S.cell_off + k] = 0;
       }
-      sort_cell(A, start, n, ln);
+      sort_cell<2>(A, start, n, ln, rows_fit(S, A.lcap));
     }
     if (!team_sync<RES>(c)) return false;
     if (rows_fit(S, A.lcap)) {

@@ -242,3 +242,33 @@ def test_noalloc_sizes(n, box):
         return
     assert np.abs(f - o.force).max() <= 1e-12 * np.abs(o.force).max()
     assert np.abs(e - o.epot_atoms).max() <= 1e-12 * np.abs(o.epot_atoms).max()
+
+
+@pytest.mark.parametrize("n", [63, 64, 65, 129, 240, 256, 257, 300])
+def test_crowded_cells(n):
+    """A cell of n atoms (every one within a cut-off of the others), at the
+    edges of the cell sort's paths: the pairs are all pairs within the list
+    cut-off, in the oracle's order where its rows (256 entries) hold them."""
+    from oracle import oracle as O
+    rng = np.random.default_rng(n)
+    pos = np.concatenate([rng.uniform(10.5, 13.5, (n, 3)), rng.uniform(0.0, 64.0, (1000, 3))])
+    s = gems.System(pos, np.ones(len(pos)))
+    s.set_box((64.0,) * 3, (True,) * 3)
+    s.set_skin(0.3)
+    s.set_lj(1.0, 0.05, 5.3)
+    s.interact()
+    d = pos[:, None] - pos[None]
+    d -= 64.0 * np.rint(d / 64.0)
+    near = (d ** 2).sum(-1) < 5.6 ** 2
+    np.fill_diagonal(near, False)
+    i, j = np.nonzero(near)
+    assert np.array_equal(s.pair_set(), i * len(pos) + j)
+    if n <= 240:
+        o = O.System(pos, np.ones(len(pos)))
+        o.set_box((64.0,) * 3, (True,) * 3)
+        o.set_skin(0.3)
+        o.set_lj(1.0, 0.05, 5.3)
+        o.interact()
+        (nn, a), (mm, b) = s.neighbour_list(), o.neighbour_list()
+        assert np.array_equal(nn, mm)
+        assert all(np.array_equal(a[:c, k], b[:c, k]) for k, c in enumerate(nn))
