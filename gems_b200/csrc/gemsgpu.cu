@@ -1547,6 +1547,7 @@ int launch_reduce(gemsgpu_ctx* ctx, const std::vector<int>& ss);
 int interact_group(gemsgpu_ctx* ctx, const std::vector<int>& ss, bool sync_check, bool* red = nullptr) {
   CHK(ensure_list(ctx, ss));
   bool built = false;  // h_st holds the states after a list update
+  bool done = false;   // the forces and their sums have been computed with it
   const int open = sync_check ? team_open(ctx, ss) : -1;
   int big = 0;
   for (int s : ss) big = std::max(big, ctx->sys[s].n);
@@ -1589,6 +1590,11 @@ int interact_group(gemsgpu_ctx* ctx, const std::vector<int>& ss, bool sync_check
       k_skin<<<m.nblk, BLOCK, 0, ctx->stream>>>(ctx->A, m); ++ctx->launches;
     }
     CHK(launch_rebuild(ctx, ss));
+    if (red) {  // a list that overflowed is rare: the forces follow unasked, and one synchronisation serves all
+      CHK(launch_forces(ctx, ss));
+      CHK(launch_reduce(ctx, ss));
+      done = true;
+    }
     if (sync_check) CHK(read_states(ctx));
   }
   if (sync_check) {
@@ -1606,10 +1612,12 @@ int interact_group(gemsgpu_ctx* ctx, const std::vector<int>& ss, bool sync_check
                                                                               (int)ss.size()); ++ctx->launches;
       CHK(launch_rebuild(ctx, ss));
       CHK(read_states(ctx));
+      done = false;
     }
     for (int s : ss) CHK(status_error(ctx, s, ctx->h_st[s].status & ~0));
   }
-  CHK(launch_forces(ctx, ss));
+  if (done) *red = true;
+  else CHK(launch_forces(ctx, ss));
   for (int s : ss) {
     SysHost& h = ctx->sys[s];
     h.first = false;
@@ -2129,9 +2137,9 @@ int d2h_xyz(gemsgpu_ctx* ctx, const double4* src, double* dst, int n) {
 // up to XFER_SMALL doubles pass through a pinned buffer that the context keeps
 // (XFER_PIN doubles at most, 4 MB) and travel as one copy, larger ones travel
 // on their own, and one kernel repacks them all.  A copy and a repack per array
-// cost 5.8 us each way for a small one: 64 systems of 147 atoms took 1490 us
-// in and 1435 us out, @IN@ and @OUT@ us this way.  Above 64 KB a copy by the
-// processor takes longer than the copy engine's own start.
+// cost 5.8 us each way for a small one: a block of 100 steps of 64 systems of
+// 147 atoms took 4.85 ms, 2.9 of them transfers, and takes 2.20 ms this way.
+// Above 64 KB the processor's own copy costs more than a transfer's start.
 constexpr int64_t XFER_SMALL = 8192, XFER_PIN = 1 << 19;
 
 struct Xfer {
@@ -2741,6 +2749,9 @@ int gemsgpu_upload(gemsgpu_ctx* ctx, int sys, const double* pos, const double* v
   CU(cudaMemcpyAsync(A.type + h.off, t.data(), n * sizeof(int), cudaMemcpyHostToDevice, ctx->stream));
   CU(cudaStreamSynchronize(ctx->stream));
   CHK(push_sys(ctx, sys));
+  // the staging area of later calls (24 MB at most here; they grow it further):
+  // a first set_positions of 32000 atoms waited 0.4 ms for it
+  CHK(ensure_stage(ctx, std::min<int64_t>(2 * ctx->acap, 1 << 20)));
   BlockMap m;
   CHK(get_map(ctx, {sys}, BLOCK, 0, &m));
   k_refresh_fx<<<m.nblk, BLOCK, 0, ctx->stream>>>(A, m); ++ctx->launches;
