@@ -272,3 +272,34 @@ def test_crowded_cells(n):
         (nn, a), (mm, b) = s.neighbour_list(), o.neighbour_list()
         assert np.array_equal(nn, mm)
         assert all(np.array_equal(a[:c, k], b[:c, k]) for k, c in enumerate(nn))
+
+
+@pytest.mark.parametrize("cells,pbc", [((14, 14, 13), (True, True, True)), ((16, 16, 16), (True, False, True)),
+                                       ((21, 21, 21), (True, True, True)), ((6, 30, 20), (True, True, False)),
+                                       ((6, 30, 20), (True, True, True))])
+def test_sparse_force_lists(cells, pbc):
+    """Force lists of sparse cells (one thread, three or nine per atom; three
+    cells a side; open faces): forces equal the oracle's, on the first list and
+    on one built after every atom has moved, and the list is the oracle's then.
+    1e-11 of the largest force: sums of 100 terms of 1e-16 and their
+    cancellation."""
+    from oracle import oracle as O
+    rng = np.random.default_rng(sum(cells))
+    g = np.stack(np.meshgrid(*[np.arange(c) for c in cells], indexing="ij"), -1).reshape(-1, 3)
+    L = tuple(1.6 * c for c in cells)
+    pos = (g + 0.5) * 1.6 + rng.uniform(-0.15, 0.15, g.shape)
+    o, s = O.System(pos, np.ones(len(pos))), gems.System(pos, np.ones(len(pos)))
+    for q in (o, s):
+        q.set_box(L, pbc)
+        q.set_skin(0.3)
+        q.set_lj(1.0, 1.0, 2.5)
+    for shift in (0.0, 0.25):
+        x = pos + np.where(rng.random(pos.shape) < 0.5, shift, -shift)
+        o.set_pos(x)
+        s.set_pos(x)
+        o.interact()
+        s.interact()
+        assert np.abs(s.force - o.force).max() <= 1e-11 * np.abs(o.force).max()
+        (nn, a), (mm, b) = s.neighbour_list(), o.neighbour_list()
+        assert np.array_equal(nn, mm)
+        assert all(np.array_equal(a[:c, k], b[:c, k]) for k, c in enumerate(nn))
