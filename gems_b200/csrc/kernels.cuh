@@ -532,9 +532,10 @@ __device__ __forceinline__ void rank_cell(const Arena& A, int start, int n, int 
     }
 }
 
-// one warp orders the n atoms of the cell whose atoms start at `start`; cells
-// of more than 64 atoms occur where a moving box leaves atoms outside its grid
-// (lane 0 alone took 50 us for one: 32000 atoms under a piston)
+// one warp orders the n atoms of the cell whose atoms start at `start`: by
+// rank, up to 32 RMAX atoms, beyond that by lane 0's insertion sort.  (10 us
+// for the cells of a rebuild of the 8 x 32k Au batch, 15 atoms each, where
+// only the first branch runs; crowded cells have not been timed.)
 template <int RMAX>
 __device__ __forceinline__ void sort_cell(const Arena& A, int start, int n, int ln, bool rec) {
   if (n <= 64) {
